@@ -23,7 +23,8 @@ namespace dgmr {
 
 constexpr unsigned kRayWarps = 4; // rays per block
 constexpr unsigned kRayRounds = 4; // 4 x 32 lanes >= 128 borders
-constexpr unsigned kRayMaskRegs = 4; // ray masks kept in registers: 4 x 32 batches of 32 entries
+template <class T>
+constexpr unsigned kRayList = sizeof(T) == 4 ? 1024 : 512; // list entries a ray can use that its warp keeps (RayList; 48 KB per block)
 
 // A ray's section set lives in shared memory, once per warp: lane 0 inserts,
 // every lane reads it after a __syncwarp (kept per lane, the 32 identical
@@ -34,6 +35,7 @@ struct RayWarpShared {
     Bin<T> bins[kSmallSteps]; // forward: (r, g, b, exp(-mass)); backward: (r, g, b, mass)
     SectionSet<kLargeSteps, T> sec;
     Section<T> pieces[2 * kLargeSteps + 1]; // warp_put: the merged sections of one insertion
+    uint16_t use[kRayList<T>]; // RayList
 };
 
 template <class T>
@@ -44,36 +46,27 @@ struct RayWarpSharedBwd {
     int32_t queue[32]; // pass 3: list entries waiting for a lane
     SectionSet<kLargeSteps, T> sec;
     Section<T> pieces[2 * kLargeSteps + 1];
+    uint16_t use[kRayList<T>]; // RayList
 };
 
 static_assert(kLargeSteps <= 16, "warp_put moves the kept sections on lanes 0-15 and writes pieces on lanes 16-31");
 
-// The gates of both passes (see ray_can_use) as a 32-bit mask per batch of 32
-// list entries, held in registers: lane l keeps the masks of batches l, l+32,
-// l+64, l+96.  Batches past that get every entry (the gates are re-checked).
-struct WarpRayMasks {
-    uint32_t r[kRayMaskRegs];
-    __device__ __forceinline__ uint32_t get(unsigned i) const
-    {
-        if (i >= 32 * kRayMaskRegs)
-            return 0xffffffffu;
-        const unsigned q = i >> 5;
-        uint32_t v = r[0];
-#pragma unroll
-        for (unsigned k = 1; k < kRayMaskRegs; ++k)
-            if (q == k)
-                v = r[k];
-        return __shfl_sync(0xffffffffu, v, int(i & 31u));
-    }
-    __device__ __forceinline__ void set(unsigned i, uint32_t m, unsigned lane)
-    {
-        if (i >= 32 * kRayMaskRegs || (i & 31u) != lane)
-            return;
-#pragma unroll
-        for (unsigned k = 0; k < kRayMaskRegs; ++k)
-            if ((i >> 5) == k)
-                r[k] = m;
-    }
+// The entries of the tile's list that the ray can use (ray_can_use), as offsets
+// into the list, packed in list order: `use` holds the first n of them, found
+// in the list's first `raw` entries; entries from `raw` on are not packed (the
+// list has more than kRayList usable entries, or offsets past 16 bits) and
+// every pass tests them.  A warp reads the packed entries 32 at a time, one per
+// lane, then the rest of the list.
+// The passes of a large step intersect every usable entry again, and a ray can
+// use few of its tile's entries: 175 of 545 at 100k Gaussians, 512^2, spread
+// over 23 of the list's 23.6 batches of 32; 282 of 9500 in 151 of 298 batches at
+// 64^2.  Packed, they fill 6 and 9 batches.  Against a bit mask per batch of 32
+// (one sparse batch after the other): forward + backward 53.7 -> 40.4 ms at
+// 100k, 512^2 (with the step store), 81.2 -> 38.8 ms for 16 batched 64^2 views,
+// forward 2.43 -> 1.88 ms at 10k, 256^2.
+struct RayList {
+    const uint16_t* use;
+    uint32_t n, raw;
 };
 
 __device__ __forceinline__ uint32_t lanes_below(int n) { return n >= 32 ? 0xffffffffu : ((1u << n) - 1u); }
@@ -136,25 +129,41 @@ __device__ __forceinline__ bool ray_pixel(const Frames& frames, const uint32_t* 
     return *px < cam.W && *py < cam.H;
 }
 
-// pass 0: the ray's masks (one intersection per list entry, lane-parallel)
+// pass 0: the ray's usable entries (one intersection per list entry, lane-parallel)
 template <class T>
-__device__ __forceinline__ WarpRayMasks warp_ray_masks(const VmMarch<T>& a, int32_t b, int32_t e, V3<T> o, V3<T> d, unsigned lane)
+__device__ __forceinline__ RayList warp_ray_list(uint16_t* use, const VmMarch<T>& a, int32_t b, int32_t e, V3<T> o, V3<T> d, unsigned lane)
 {
-    WarpRayMasks rm;
-#pragma unroll
-    for (unsigned k = 0; k < kRayMaskRegs; ++k)
-        rm.r[k] = 0u;
-    unsigned i = 0;
-    for (int32_t base = b; base < e && i < 32 * kRayMaskRegs; base += 32, ++i) {
-        const int32_t k = base + int32_t(lane);
+    uint32_t n = 0, raw = 0;
+    const uint32_t len = uint32_t(e - b);
+    for (; raw < len && raw + 32u <= 0x10000u; raw += 32) {
+        const uint32_t k = raw + lane;
         bool can = false;
-        if (k < e) {
-            const RayEntry<T> en = load_entry(a, k);
+        if (k < len) {
+            const RayEntry<T> en = load_entry(a, b + int32_t(k));
             can = ray_can_use(intersect_with_ray_inv_C(en.mu, en.Q, o, d), en.mass);
         }
-        rm.set(i, __ballot_sync(0xffffffffu, can), lane);
+        const uint32_t m = __ballot_sync(0xffffffffu, can);
+        if (n + uint32_t(__popc(m)) > kRayList<T>)
+            break;
+        if (can)
+            use[n + uint32_t(__popc(m & lanes_below(int(lane))))] = uint16_t(k);
+        n += uint32_t(__popc(m));
     }
-    return rm;
+    __syncwarp();
+    return RayList { use, n, min(raw, len) };
+}
+
+// The list entry of the lane in batch t of a pass (-1: none), and how many batches a pass has.
+__device__ __forceinline__ uint32_t ray_batches(const RayList& rl, int32_t b, int32_t e) { return (rl.n + 31u) / 32u + (uint32_t(e - b) - rl.raw + 31u) / 32u; }
+__device__ __forceinline__ int32_t ray_entry(const RayList& rl, int32_t b, int32_t e, uint32_t t, unsigned lane)
+{
+    const uint32_t packed = (rl.n + 31u) / 32u;
+    if (t < packed) {
+        const uint32_t j = 32u * t + lane;
+        return j < rl.n ? b + int32_t(rl.use[j]) : -1;
+    }
+    const int32_t k = b + int32_t(rl.raw + 32u * (t - packed) + lane);
+    return k < e ? k : -1;
 }
 
 } // namespace dgmr
@@ -308,12 +317,12 @@ __device__ __forceinline__ void warp_sample_positions(const SectionSet<kLargeSte
     __syncwarp();
 }
 
-// Pass 1 (vol_marcher_forward.cu:351-403): the masked entries of a batch are
+// Pass 1 (vol_marcher_forward.cu:351-403): a batch of the ray's entries is
 // intersected lane-parallel, then walked in list order and inserted into the
 // warp's section set (in shared memory, warp_put), which every lane reads.
 template <PutMode kPut = PutMode::Inline, class T>
 __device__ __forceinline__ void warp_collect(SectionSet<kLargeSteps, T>& sec, Section<T>* pieces, const VmMarch<T>& a, int32_t b, int32_t e, V3<T> o,
-    V3<T> d, const WarpRayMasks& rm, unsigned lane)
+    V3<T> d, const RayList& rl, unsigned lane)
 {
     if (a.cs.n > 0) {
         if (lane == 0)
@@ -322,15 +331,14 @@ __device__ __forceinline__ void warp_collect(SectionSet<kLargeSteps, T>& sec, Se
         __syncwarp();
         return;
     }
-    unsigned i = 0;
-    for (int32_t base = b; base < e; base += 32, ++i) {
-        uint32_t m = rm.get(i) & lanes_below(e - base);
-        if (!m)
-            continue;
+    const uint32_t batches = ray_batches(rl, b, e);
+    for (uint32_t t = 0; t < batches; ++t) {
+        const int32_t entry = ray_entry(rl, b, e, t, lane);
+        uint32_t m = __ballot_sync(0xffffffffu, entry >= 0);
         T depth = T(0), s0 = T(0), s1 = T(0), dt = T(0);
         bool ok = false;
-        if ((m >> lane) & 1u) {
-            const RayEntry<T> en = load_entry(a, base + int32_t(lane));
+        if (entry >= 0) {
+            const RayEntry<T> en = load_entry(a, entry);
             const Gauss1d<T> g = intersect_with_ray_inv_C(en.mu, en.Q, o, d);
             const T sd = dgmr_fm::sqrt_f(g.C);
             depth = a.depths[en.id];
@@ -398,7 +406,7 @@ __device__ __forceinline__ void warp_bins(Bin<T> (&acc)[kRayRounds], const T* bo
     }
 }
 
-// The 1-D Gaussian of a masked entry if it reaches the bins (the early-outs of
+// The 1-D Gaussian of a usable entry if it reaches the bins (the early-outs of
 // math.h:442-459); the same test in the forward and backward.
 template <class T>
 __device__ __forceinline__ bool warp_entry_on_bins(const RayEntry<T>& en, V3<T> o, V3<T> d, const T* borders, Gauss1d<T>* g_out, T* sd_out, T* inv_sd_out,
@@ -423,21 +431,20 @@ __device__ __forceinline__ bool warp_entry_on_bins(const RayEntry<T>& en, V3<T> 
 // over the lanes; returns how many Gaussians filled the bins (the same on every lane)
 template <class T>
 __device__ __forceinline__ unsigned warp_fill(Bin<T> (&acc)[kRayRounds], const T* borders, const VmMarch<T>& a, int32_t b, int32_t e, V3<T> o, V3<T> d,
-    const WarpRayMasks& rm, unsigned lane)
+    const RayList& rl, unsigned lane)
 {
 #pragma unroll
     for (unsigned r = 0; r < kRayRounds; ++r)
         acc[r] = Bin<T> { T(0), T(0), T(0), T(0) };
-    unsigned i = 0, fills = 0;
-    for (int32_t base = b; base < e; base += 32, ++i) {
-        const uint32_t m = rm.get(i) & lanes_below(e - base);
-        if (!m)
-            continue;
+    unsigned fills = 0;
+    const uint32_t batches = ray_batches(rl, b, e);
+    for (uint32_t t = 0; t < batches; ++t) {
+        const int32_t entry = ray_entry(rl, b, e, t, lane);
         T centre = T(0), inv_sd = T(0), mor = T(0);
         V3<T> rgb = { T(0), T(0), T(0) };
         bool ok = false;
-        if ((m >> lane) & 1u) {
-            const RayEntry<T> en = load_entry(a, base + int32_t(lane));
+        if (entry >= 0) {
+            const RayEntry<T> en = load_entry(a, entry);
             Gauss1d<T> g;
             T sd;
             ok = warp_entry_on_bins(en, o, d, borders, &g, &sd, &inv_sd, &mor);
@@ -485,7 +492,7 @@ __global__ void __launch_bounds__(kRayWarps * 32, sizeof(T) == 4 ? 8 : 2) k_vm_m
     const V3<T> o = { cam.campos[0], cam.campos[1], cam.campos[2] };
     const V3<T> d = pixel_dir(cam, px, py);
     const int32_t b = a.ranges[2 * tile], e = a.ranges[2 * tile + 1];
-    const WarpRayMasks rm = warp_ray_masks(a, b, e, o, d, lane);
+    const RayList rl = warp_ray_list(sm.use, a, b, e, o, d, lane);
     V3<T> colour = { T(0), T(0), T(0) };
     T tr = T(1);
     T start = T(0);
@@ -501,7 +508,7 @@ __global__ void __launch_bounds__(kRayWarps * 32, sizeof(T) == 4 ? 8 : 2) k_vm_m
         if (lane == 0)
             sec.reset(start);
         __syncwarp();
-        warp_collect(sec, sm.pieces, a, b, e, o, d, rm, lane);
+        warp_collect(sec, sm.pieces, a, b, e, o, d, rl, lane);
         warp_sample_positions(sec, sm.borders, lane);
         if (step < a.store_steps) {
             // keep this step's samples for the backward (coalesced: 32 lanes x 4 rounds)
@@ -514,7 +521,7 @@ __global__ void __launch_bounds__(kRayWarps * 32, sizeof(T) == 4 ? 8 : 2) k_vm_m
                 a.store_sections[size_t(step) * rays + ray] = int32_t(sec.n);
         }
         Bin<T> acc[kRayRounds];
-        fills += warp_fill(acc, sm.borders, a, b, e, o, d, rm, lane);
+        fills += warp_fill(acc, sm.borders, a, b, e, o, d, rl, lane);
         warp_store_bins(sm.bins, acc, lane, a.mode != DGMR_RENDER_BINS);
         if (a.mode == DGMR_RENDER_FULL) {
             // math.h:412-428, identical on every lane
@@ -603,16 +610,15 @@ __device__ __noinline__ void lane_grad_entry(const VmMarch<T>& a, int32_t k, con
 // queued (its atomics would all be skipped as zeros).
 template <class T>
 __device__ __forceinline__ void warp_grad(const Bin<T>* gbins, const T* borders, int32_t* queue, const VmMarch<T>& a, int32_t b, int32_t e, V3<T> o, V3<T> d,
-    const WarpRayMasks& rm, unsigned lane, int live_end)
+    const RayList& rl, unsigned lane, int live_end)
 {
-    unsigned i = 0, fill = 0;
-    for (int32_t base = b; base < e; base += 32, ++i) {
-        const uint32_t m = rm.get(i) & lanes_below(e - base);
-        if (!m)
-            continue;
+    unsigned fill = 0;
+    const uint32_t batches = ray_batches(rl, b, e);
+    for (uint32_t t = 0; t < batches; ++t) {
+        const int32_t entry = ray_entry(rl, b, e, t, lane);
         bool ok = false;
-        if ((m >> lane) & 1u) {
-            const RayEntry<T> en = load_entry(a, base + int32_t(lane));
+        if (entry >= 0) {
+            const RayEntry<T> en = load_entry(a, entry);
             Gauss1d<T> g;
             T sd, inv_sd, mor;
             ok = warp_entry_on_bins(en, o, d, borders, &g, &sd, &inv_sd, &mor);
@@ -627,7 +633,7 @@ __device__ __forceinline__ void warp_grad(const Bin<T>* gbins, const T* borders,
         if (ok) {
             const unsigned slot = fill + unsigned(__popc(okm & lanes_below(int(lane))));
             if (slot < 32)
-                queue[slot] = base + int32_t(lane);
+                queue[slot] = entry;
         }
         __syncwarp();
         if (fill + n_ok >= 32) {
@@ -638,7 +644,7 @@ __device__ __forceinline__ void warp_grad(const Bin<T>* gbins, const T* borders,
             if (ok) {
                 const unsigned slot = fill + unsigned(__popc(okm & lanes_below(int(lane))));
                 if (slot >= 32)
-                    queue[slot - 32] = base + int32_t(lane);
+                    queue[slot - 32] = entry;
             }
             __syncwarp();
             fill = left;
@@ -669,7 +675,7 @@ __global__ void __launch_bounds__(kRayWarps * 32, sizeof(T) == 4 ? 6 : 2) k_vm_m
     const V3<T> o = { cam.campos[0], cam.campos[1], cam.campos[2] };
     const V3<T> d = pixel_dir(cam, px, py);
     const int32_t b = a.ranges[2 * tile], e = a.ranges[2 * tile + 1];
-    const WarpRayMasks rm = warp_ray_masks(a, b, e, o, d, lane);
+    const RayList rl = warp_ray_list(sm.use, a, b, e, o, d, lane);
     const size_t pix = size_t(py) * cam.W + px;
     const size_t plane = size_t(cam.W) * cam.H;
     const T* fb = frames.fb(view, a);
@@ -700,12 +706,12 @@ __global__ void __launch_bounds__(kRayWarps * 32, sizeof(T) == 4 ? 6 : 2) k_vm_m
             if (lane == 0)
                 sec.reset(start);
             __syncwarp();
-            warp_collect<PutMode::Call>(sec, sm.pieces, a, b, e, o, d, rm, lane);
+            warp_collect<PutMode::Call>(sec, sm.pieces, a, b, e, o, d, rl, lane);
             warp_sample_positions(sec, sm.borders, lane);
             n_sections = int(sec.n);
         }
         Bin<T> acc[kRayRounds];
-        warp_fill(acc, sm.borders, a, b, e, o, d, rm, lane);
+        warp_fill(acc, sm.borders, a, b, e, o, d, rl, lane);
         warp_store_bins(sm.bins, acc, lane, false);
         // grad/math.h:529-557, identical on every lane; lane 0 stores the bin adjoints
         unsigned k = 0;
@@ -735,7 +741,7 @@ __global__ void __launch_bounds__(kRayWarps * 32, sizeof(T) == 4 ? 6 : 2) k_vm_m
             if (lane == 0)
                 sm.gbins[k] = Bin<T> { T(0), T(0), T(0), T(0) };
         __syncwarp();
-        warp_grad(sm.gbins, sm.borders, sm.queue, a, b, e, o, d, rm, lane, live_end);
+        warp_grad(sm.gbins, sm.borders, sm.queue, a, b, e, o, d, rl, lane, live_end);
         const bool done = n_sections == 0 || tr < T(1.f / 255.f);
         start = sm.borders[kSmallSteps - 1];
         __syncwarp();

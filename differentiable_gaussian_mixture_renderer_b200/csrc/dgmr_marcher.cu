@@ -251,11 +251,11 @@ inline size_t step_store_bytes(uint32_t n_rays, uint32_t steps, size_t elem)
 // step only act on a Gaussian that passes its gate -- pass 1's (mass on the
 // ray in (1/255, 1000], positive variance, finite centre) or pass 2's
 // (gaussian_on_ray) -- and the gates depend on the ray alone, not on the
-// step.  So a first pass over the tile records, per ray and per batch of list
-// entries, a mask of the entries that pass either gate, and the large steps
-// only intersect those.  Pass 1's depth break also only needs them: the list
-// is in depth order, so the first entry with depth > end of the section set
-// that is skipped here would be followed by a masked entry with a depth at
+// step.  So a first pass over the tile packs, per ray, the list entries that
+// pass either gate (RayList), and the large steps only intersect those.
+// Pass 1's depth break also only needs them: the list is in depth order, so
+// the first entry with depth > end of the section set that is skipped here
+// would be followed by a packed entry with a depth at
 // least as large, checked against the same end.  The results are identical;
 // the per-step cost drops from the tile's list to the ray's own Gaussians.
 template <class T>
