@@ -34,7 +34,7 @@ constexpr unsigned kRayList = sizeof(T) == 4 ? 1024 : 512; // list entries a ray
 template <class T>
 struct RayWarpShared {
     T borders[kSmallSteps];
-    Bin<T> bins[kSmallSteps]; // forward: (r, g, b, exp(-mass)); backward: (r, g, b, mass)
+    Bin<T> bins[kSmallSteps]; // (r, g, b, exp(-mass))
     SectionSet<kLargeSteps, T> sec;
     Section<T> pieces[2 * kLargeSteps + 1]; // warp_put: the merged sections of one insertion
     uint16_t use[kRayList<T>]; // RayList
@@ -47,7 +47,10 @@ struct RayWarpSharedBwd {
     Bin<T> gbins[kSmallSteps]; // bin adjoints
     int32_t queue[32]; // pass 3: list entries waiting for a lane
     SectionSet<kLargeSteps, T> sec;
-    Section<T> pieces[2 * kLargeSteps + 1];
+    union {
+        Section<T> pieces[2 * kLargeSteps + 1]; // pass 1
+        T inv_t[kSmallSteps]; // warp_peel: 1 / exp(-mass) of each bin
+    };
     uint16_t use[kRayList<T>]; // RayList
 };
 
@@ -486,7 +489,7 @@ __device__ __forceinline__ unsigned warp_fill(Bin<T> (&acc)[kRayRounds], const T
     return fills;
 }
 
-// bins to shared memory in order (.m = exp(-mass) for the blend, the mass itself for the peel)
+// bins to shared memory in order (.m = exp(-mass), or the mass itself for the Bins mode)
 template <class T>
 __device__ __forceinline__ void warp_store_bins(Bin<T>* bins, const Bin<T> (&acc)[kRayRounds], unsigned lane, bool transmittance)
 {
@@ -678,6 +681,71 @@ __device__ __forceinline__ void warp_grad(const Bin<T>* gbins, const T* borders,
     __syncwarp();
 }
 
+// The colour peel of one large step and the bin adjoints (grad/math.h:529-557),
+// from the lane's bins 32 r + lane; returns one past the bin where the ray
+// stopped.  exp(-mass) and its reciprocal are computed by the bin's own lane,
+// and so are the adjoints, from the colour and transmittance that the lane
+// takes out of the walk at its bin.  Only the walk itself (the two products and
+// the subtraction that chain the bins) runs on every lane, and only over the
+// bins that hold any mass: an empty bin changes neither the colour nor the
+// transmittance, and its adjoint is never read (no Gaussian reached it with
+// the mass that pass 3 asks for).  The same operations, in the same order.
+// Against the walk over every bin with the exp and the division on every lane:
+// forward + backward 45.1 -> 41.3 ms at 100k, 512^2 (mean of four cameras), 1.86
+// -> 1.63 ms in float64 at 4k, 97x65.
+template <class T>
+__device__ __forceinline__ int warp_peel(Bin<T>* gbins, Bin<T>* bins, T* inv_t, const Bin<T> (&acc)[kRayRounds], V3<T> gc, T gt, T final_T, V3<T>& colour,
+    T& tr, unsigned lane)
+{
+    T tks[kRayRounds], invs[kRayRounds];
+#pragma unroll
+    for (unsigned r = 0; r < kRayRounds; ++r) {
+        tks[r] = dgmr_fm::exp_f(-acc[r].m);
+        invs[r] = min_f(T(255), T(1) / tks[r]);
+        bins[32 * r + lane] = Bin<T> { acc[r].r, acc[r].g, acc[r].b, tks[r] };
+        inv_t[32 * r + lane] = invs[r];
+    }
+    __syncwarp();
+    int live_end = int(kBins);
+#pragma unroll
+    for (unsigned r = 0; r < kRayRounds; ++r) {
+        Bin<T> gb = { T(0), T(0), T(0), T(0) };
+        uint32_t held = __ballot_sync(0xffffffffu, acc[r].m != T(0));
+        if (live_end == int(kBins) && held) {
+            T my_tr = T(0);
+            V3<T> my_colour = { T(0), T(0), T(0) };
+            while (held) {
+                const int j = __ffs(int(held)) - 1;
+                held &= held - 1u;
+                const Bin<T> bk = bins[32 * r + j];
+                const T inv_tk = inv_t[32 * r + j];
+                colour.x = (colour.x - bk.r) * inv_tk;
+                colour.y = (colour.y - bk.g) * inv_tk;
+                colour.z = (colour.z - bk.b) * inv_tk;
+                if (int(lane) == j) {
+                    my_tr = tr;
+                    my_colour = colour;
+                }
+                tr = tr * bk.m;
+                if (tr < T(1. / 255.)) {
+                    live_end = int(32 * r) + j + 1;
+                    break;
+                }
+            }
+            if (my_tr != T(0)) {
+                gb.r = my_tr * gc.x;
+                gb.g = my_tr * gc.y;
+                gb.b = my_tr * gc.z;
+                const T g_tk = (final_T * invs[r]) * gt + dot3(gc, my_colour) * my_tr;
+                gb.m = T(0) - g_tk * tks[r];
+            }
+        }
+        gbins[32 * r + lane] = gb;
+    }
+    __syncwarp();
+    return live_end;
+}
+
 // vol_marcher_backward.cu:115-319 with one warp per ray
 template <class T, class Frames>
 __global__ void __launch_bounds__(kRayWarps * 32, sizeof(T) == 4 ? 6 : 2) k_vm_march_warp_bwd(VmMarch<T> a, const __grid_constant__ Frames frames,
@@ -733,35 +801,7 @@ __global__ void __launch_bounds__(kRayWarps * 32, sizeof(T) == 4 ? 6 : 2) k_vm_m
         }
         Bin<T> acc[kRayRounds];
         warp_fill(acc, sm.borders, a, b, e, o, d, rl, lane);
-        warp_store_bins(sm.bins, acc, lane, false);
-        // grad/math.h:529-557, identical on every lane; lane 0 stores the bin adjoints
-        unsigned k = 0;
-        for (; k < kBins; ++k) {
-            const Bin<T> bk = sm.bins[k];
-            Bin<T> gb;
-            gb.r = tr * gc.x;
-            gb.g = tr * gc.y;
-            gb.b = tr * gc.z;
-            const T tk = dgmr_fm::exp_f(-bk.m);
-            const T inv_tk = min_f(T(255), T(1) / tk);
-            colour.x = (colour.x - bk.r) * inv_tk;
-            colour.y = (colour.y - bk.g) * inv_tk;
-            colour.z = (colour.z - bk.b) * inv_tk;
-            const T g_tk = (final_T * inv_tk) * gt + dot3(gc, colour) * tr;
-            gb.m = T(0) - g_tk * tk;
-            if (lane == 0)
-                sm.gbins[k] = gb;
-            tr = tr * tk;
-            if (tr < T(1. / 255.)) {
-                ++k;
-                break;
-            }
-        }
-        const int live_end = int(k);
-        for (; k < kBins; ++k)
-            if (lane == 0)
-                sm.gbins[k] = Bin<T> { T(0), T(0), T(0), T(0) };
-        __syncwarp();
+        const int live_end = warp_peel(sm.gbins, sm.bins, sm.inv_t, acc, gc, gt, final_T, colour, tr, lane);
         warp_grad(sm.gbins, sm.borders, sm.queue, a, b, e, o, d, rl, lane, live_end);
         const bool done = n_sections == 0 || tr < T(1.f / 255.f);
         start = sm.borders[kSmallSteps - 1];
