@@ -11,6 +11,7 @@
 #include "dgmr_batch.cuh"
 #include "dgmr_binning.cuh"
 #include "dgmr_device_grad.cuh"
+#include "dgmr_f32x2.cuh"
 
 namespace dgmr {
 
@@ -28,7 +29,7 @@ struct SplatLayout {
     int32_t* ranges;
     float* final_T;
     int32_t* n_contrib;
-    double* grad_acc; // [N,9]: xy(2) conic(3) opacity rgb(3), summed over pixels in double
+    double* grad_acc; // [N,9]: moments of d/dq (dx, dy, dx^2, dx dy, dy^2), opacity, rgb(3), summed over pixels in double
     float4* blend_rec; // [N,2]: (x, y, a, c), (2b, opacity, q_cut, 0) -- the blend's 32-byte record
     uint32_t* tile_order; // [tiles] launch order of the per-tile kernels, heaviest first
     uint32_t* tile_cost; // [tiles] predicted blend cost of each tile as a bucket, 0 = heaviest
@@ -422,20 +423,22 @@ void launch_blend(int side, uint32_t n_tiles, const int32_t* ranges, const uint3
     note_launch();
 }
 
-// Sums of 9 per-lane values over a warp, scattered: halve the slots each lane
-// holds at every butterfly level (16 -> 8 -> 4 -> 2 -> 1, the upper half kept
-// by the lanes whose level bit is set), then add the partner's copy.  Lane l
-// returns the warp total of slot 8 b4 + 4 b3 + 2 b2 + b1 (b = the bits of l;
-// slots 9..15 are zero).
-__device__ __forceinline__ float warp_reduce_scatter9(const float (&v)[9], int lane)
+// Sums of 9 per-lane values over a warp, scattered.  Slots 0..7: halve the
+// slots each lane holds at every butterfly level (8 -> 4 -> 2 -> 1, the upper half
+// kept by the lanes whose level bit is set), then add the partners left; slot 8: a
+// plain butterfly.  Lane l returns the warp total of slot 4 b4 + 2 b3 + b2 (b =
+// the bits of l) and, in `ninth`, that of slot 8.  The last two levels add in
+// double: the terms of a long thin splat cancel, and a float sum ends at 8 lanes
+// (16 pixels).
+__device__ __forceinline__ double warp_reduce_scatter9(const float (&v)[9], int lane, double* ninth)
 {
-    float a[16];
+    float a[8], last = v[8];
 #pragma unroll
-    for (int q = 0; q < 16; ++q)
-        a[q] = q < 9 ? v[q] : 0.f;
+    for (int q = 0; q < 8; ++q)
+        a[q] = v[q];
 #pragma unroll
-    for (int half = 8; half >= 1; half >>= 1) {
-        const int bit = half * 2; // the xor distance: 16, 8, 4, 2
+    for (int half = 4; half >= 1; half >>= 1) {
+        const int bit = half * 4; // the xor distance: 16, 8, 4
         const bool upper = (lane & bit) != 0;
 #pragma unroll
         for (int q = 0; q < half; ++q) {
@@ -443,178 +446,292 @@ __device__ __forceinline__ float warp_reduce_scatter9(const float (&v)[9], int l
             const float keep = upper ? a[q + half] : a[q];
             a[q] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
         }
+        last += __shfl_xor_sync(0xffffffffu, last, bit);
     }
-    return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
+    double sum = double(a[0]), end = double(last);
+#pragma unroll
+    for (int bit = 2; bit >= 1; bit >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, bit);
+        end += __shfl_xor_sync(0xffffffffu, end, bit);
+    }
+    *ninth = end;
+    return sum;
 }
 
-// Reverse-order blend adjoint: each pixel walks its contributors back to
-// front, recovering T_i = T_{i+1} / (1 - alpha_i); per-splat gradients are
-// summed over the warp with shuffles before one atomic per value.  Tiles run
-// in the forward's launch order (heaviest predicted walk first): a tile's
-// backward walks the same list up to its last contributor.
-// The block shapes of the forward (BlendShape): with 8x8 blocks each block
-// walks only up to the last contributor of its own 64 pixels.
-// __launch_bounds__: 48 registers (for 16x16, instead of 53: five blocks per
-// SM instead of four, backward 2-3 % shorter at 1080p/1M and 200k/1024^2).
-template <int kSide, class Frames>
-__global__ void __launch_bounds__(BlendShape<kSide>::kThreads, BlendShape<kSide>::kMinBlocks) k_splat_bwd_pixels(const int32_t* __restrict__ ranges,
-    const uint32_t* __restrict__ list, const float4* __restrict__ rec, const float* __restrict__ rgb, double* __restrict__ acc,
-    const uint32_t* __restrict__ tile_order, const __grid_constant__ Frames frames)
+// Reverse-order blend adjoint.  A warp owns an 8x8 quarter of a tile and a lane
+// two of its pixels, (x, y) and (x, y + 4), as the halves of packed floats: the
+// quadratic form, the exp, the inverse blend step and the partials are one
+// packed operation for both, and a record's partials are summed over 64 pixels
+// by one warp reduction.  Each pixel walks its contributors back to front,
+// recovering T_i = T_{i+1} / (1 - alpha_i).  Per record the warp sums the
+// moments of g_q = d/dq over its pixels (g_q dx, g_q dy, g_q dx^2, g_q dx dy,
+// g_q dy^2), d/dopacity and d/drgb -- the centre's and the conic's gradients are
+// linear in the moments, which k_splat_bwd_gaussians applies to the totals -- and
+// nine lanes add one value each.  The totals over warps are double: in float,
+// the order in which the atomics of many cancelling terms land moved single
+// elements by ~1e-3 relative from run to run at 200k Gaussians, 1024^2.
+// Tiles run in the forward's launch order (heaviest predicted walk first); a
+// warp walks its tile's list only up to its own pixels' last contributor.
+//
+// Bound by instruction issue, and at the end of a launch by the longest warp's
+// serial walk: so a record's reduction is issued with the next record's body, and
+// 80 registers without spills (six blocks per SM) beat 64 with them.  Against a
+// pixel per lane, a reduction per 32 pixels and 48 registers, forward + backward
+// (mean of four cameras): 0.946 -> 0.800 ms at 200k, 1024^2; 1.323 -> 1.192 ms at
+// 1M, 1080p; 6.42 -> 5.47 ms for 12 batched views.
+constexpr int kBwdWarps = 4; // the quarters of a tile
+static_assert(kTile == 16, "four 8x8 quarters per tile");
+
+// The largest magnitude that the packed walk takes from a record or a pixel: the
+// half that does not use a record is multiplied by an exact zero, which needs
+// finite operands (products of two such values are finite, and so is the
+// quadratic form of such a geometry).  Others take the guarded walk.
+constexpr float kBwdPlain = 1.0e18f, kBwdPlainGeometry = 1.0e9f;
+__device__ __forceinline__ bool bwd_plain(float x, float most = kBwdPlain) { return fabsf(x) <= most; } // false for NaN
+
+struct BwdPixels {
+    F2 Tr; // transmittance in front of the records walked so far
+    F2 a0, a1, a2; // colour behind the current record
+    F2 g0, g1, g2; // image gradient
+    F2 bg; // final T times the gradient's product with the background
+    int32_t n0, n1; // contributors
+};
+
+// One record on the lane's two pixels: `use` says which of them it reaches.
+// Returns whether any partial is nonzero.  kGuarded: values may be huge or not
+// finite, and a pixel that does not use the record must not see them.
+template <bool kGuarded>
+__device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, float4 c, F2 q, float dx, F2 dy, bool use0, bool use1, float (&v)[9])
 {
-    constexpr int kThreads = BlendShape<kSide>::kThreads;
-    constexpr int kPerTile = BlendShape<kSide>::kPerTile;
-    constexpr int kWarps = kThreads / 32;
-    __shared__ float4 s_r0[kThreads]; // the blend records: (x, y, a, c), (2b, opacity, q_cut, list index as int bits)
-    __shared__ float4 s_r1[kThreads];
-    __shared__ float s_rgb[3][kThreads];
-    __shared__ uint32_t s_id[kThreads];
-    __shared__ int s_warp_tot[kWarps];
-    __shared__ int s_max;
-    const unsigned slot = blockIdx.x / kPerTile, part = blockIdx.x % kPerTile, n_tiles = gridDim.x / kPerTile;
-    const unsigned ordered = tile_order ? tile_order[slot] : slot;
-    const unsigned tile = ordered < n_tiles ? ordered : slot; // the order is a permutation of the tiles
+    const float op = r1.y;
+    float e0, e1;
+    split2(exp2_nonpos(mul2(q, f2(-0.5f))), &e0, &e1);
+    {
+        float q0, q1;
+        split2(q, &q0, &q1);
+        if (kGuarded) {
+            if (use0 && !(q0 >= -170.f && q0 <= 170.f))
+                e0 = dgmr_fm::exp_f_nonpos(-0.5f * q0);
+            if (use1 && !(q1 >= -170.f && q1 <= 170.f))
+                e1 = dgmr_fm::exp_f_nonpos(-0.5f * q1);
+        } else if (fminf(q0, q1) < -170.f) { // rounding of a long thin splat far away; q <= q_cut < 100 where it is used
+            e0 = dgmr_fm::exp_f_nonpos(-0.5f * q0);
+            e1 = dgmr_fm::exp_f_nonpos(-0.5f * q1);
+        }
+    }
+    const float og0 = op * e0, og1 = op * e1;
+    float al0 = min_f(0.99f, og0), al1 = min_f(0.99f, og1);
+    use0 = use0 && !(al0 < 1.0f / 255.0f);
+    use1 = use1 && !(al1 < 1.0f / 255.0f);
+    al0 = use0 ? al0 : 0.f;
+    al1 = use1 ? al1 : 0.f;
+    const F2 g = f2(use0 ? e0 : 0.f, use1 ? e1 : 0.f), alpha = f2(al0, al1);
+    // 1 / (1 - alpha), 1 - alpha in [0.01, 1]: the hardware's approximation and
+    // one Newton step y + y (1 - x y)
+    const float x0 = 1.f - al0, x1 = 1.f - al1;
+    float y0, y1;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(x0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(x1));
+    F2 inv = f2(y0, y1);
+    inv = fma2(inv, fma2(f2(-x0, -x1), inv, f2(1.f)), inv);
+    const F2 Tr = mul2(p.Tr, inv);
+    const F2 aT = mul2(alpha, Tr);
+    const F2 w0 = mul2(aT, p.g0), w1 = mul2(aT, p.g1), w2 = mul2(aT, p.g2);
+    const F2 neg = f2(-1.f);
+    const F2 d0 = fma2(p.a0, neg, f2(c.x)), d1 = fma2(p.a1, neg, f2(c.y)), d2 = fma2(p.a2, neg, f2(c.z));
+    const F2 dot = fma2(d2, p.g2, fma2(d1, p.g1, mul2(d0, p.g0)));
+    const F2 ga = fma2(Tr, dot, mul2(mul2(p.bg, neg), inv));
+    float ga0, ga1;
+    split2(ga, &ga0, &ga1);
+    ga0 = og0 < 0.99f ? ga0 : 0.f; // alpha = 0.99 there, whatever the opacity
+    ga1 = og1 < 0.99f ? ga1 : 0.f;
+    const F2 go = mul2(f2(ga0, ga1), g); // d/dopacity
+    const F2 gq = mul2(go, f2(-0.5f * op));
+    const F2 gy = mul2(gq, dy), gyy = mul2(gy, dy);
+    const F2 na0 = fma2(alpha, d0, p.a0), na1 = fma2(alpha, d1, p.a1), na2 = fma2(alpha, d2, p.a2);
+    const auto sum = [&](F2 t) {
+        float lo, hi;
+        split2(t, &lo, &hi);
+        if (kGuarded) {
+            lo = use0 ? lo : 0.f;
+            hi = use1 ? hi : 0.f;
+        }
+        return lo + hi;
+    };
+    const float s = sum(gq);
+    v[0] = dx * s;
+    v[1] = sum(gy);
+    v[2] = dx * v[0];
+    v[3] = dx * v[1];
+    v[4] = sum(gyy);
+    v[5] = sum(go);
+    v[6] = sum(w0);
+    v[7] = sum(w1);
+    v[8] = sum(w2);
+    if (kGuarded) {
+        if (!use0 && !use1) {
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+                v[k] = 0.f; // dx may not be finite
+        }
+        const auto pick = [&](F2& to, F2 from) {
+            float a, b, x, y;
+            split2(to, &a, &b);
+            split2(from, &x, &y);
+            to = f2(use0 ? x : a, use1 ? y : b);
+        };
+        pick(p.Tr, Tr);
+        pick(p.a0, na0);
+        pick(p.a1, na1);
+        pick(p.a2, na2);
+    } else {
+        p.Tr = Tr;
+        p.a0 = na0;
+        p.a1 = na1;
+        p.a2 = na2;
+    }
+    return use0 || use1;
+}
+
+template <class Frames>
+__global__ void __launch_bounds__(kBwdWarps * 32, 6) k_splat_bwd_pixels(const int32_t* __restrict__ ranges, const uint32_t* __restrict__ list,
+    const float4* __restrict__ rec, const float* __restrict__ rgb, double* __restrict__ acc, const uint32_t* __restrict__ tile_order,
+    const __grid_constant__ Frames frames)
+{
+    __shared__ float4 s_r0[kBwdWarps][32]; // the blend records: (x, y, a, c), (2b, opacity, q_cut, list index as int bits)
+    __shared__ float4 s_r1[kBwdWarps][32];
+    __shared__ float4 s_rgb[kBwdWarps][32]; // colour, Gaussian as int bits
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned ordered = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
+    const unsigned tile = ordered < gridDim.x ? ordered : blockIdx.x; // the order is a permutation of the tiles
     const FrameRef f = frames.frame(tile);
     if (!f.grad_fb) // a view without an image gradient (batched renders that only asked for the image)
         return;
     const unsigned W = f.W, H = f.H;
-    const unsigned tx = f.tile % f.gx, ty = f.tile / f.gx;
-    // the forward's pixel blocks: the block's pixels start at (ox, oy) of the
-    // tile, warp w covers the 8x4 block (8 (w % kRow), 4 (w / kRow)) of them
-    constexpr unsigned kRow = unsigned(kSide) / 8u;
-    const unsigned ox = unsigned(kSide) * (part % (kTile / unsigned(kSide))), oy = unsigned(kSide) * (part / (kTile / unsigned(kSide)));
-    const unsigned wb = threadIdx.x >> 5;
-    const unsigned px = tx * kTile + ox + 8u * (wb % kRow) + (threadIdx.x & 7u);
-    const unsigned py = ty * kTile + oy + 4u * (wb / kRow) + ((threadIdx.x >> 3) & 3u);
-    const bool inside = px < W && py < H;
-    const int32_t b = ranges[2 * tile];
-    const size_t pix = size_t(py) * W + px;
-    const int32_t my_n = inside ? f.n_contrib[pix] : 0;
-    if (threadIdx.x == 0)
-        s_max = 0;
-    __syncthreads();
-    atomicMax(&s_max, my_n);
-    __syncthreads();
-    const int32_t max_n = s_max;
-    float g0 = 0.f, g1 = 0.f, g2 = 0.f, Tf = 1.f;
-    if (inside) {
-        g0 = f.grad_fb[pix];
-        g1 = f.grad_fb[size_t(W) * H + pix];
-        g2 = f.grad_fb[2 * size_t(W) * H + pix];
-        Tf = f.final_T[pix];
+    const unsigned x0 = (f.tile % f.gx) * kTile + 8u * (unsigned(warp) & 1u), y0 = (f.tile / f.gx) * kTile + 8u * (unsigned(warp) >> 1);
+    const unsigned px = x0 + (unsigned(lane) & 7u), py = y0 + (unsigned(lane) >> 3);
+    const size_t plane = size_t(W) * H;
+    BwdPixels p;
+    float g[2][3], T[2], bg[2];
+    int32_t n[2];
+    bool plain = true;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const unsigned y = py + 4u * unsigned(h);
+        const bool inside = px < W && y < H;
+        const size_t pix = size_t(y) * W + px;
+        n[h] = inside ? f.n_contrib[pix] : 0;
+        T[h] = inside ? f.final_T[pix] : 1.f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            g[h][c] = inside ? f.grad_fb[c * plane + pix] : 0.f;
+            plain = plain && bwd_plain(g[h][c]);
+        }
+        bg[h] = T[h] * ((f.bg0 * g[h][0] + f.bg1 * g[h][1]) + f.bg2 * g[h][2]);
+        plain = plain && bwd_plain(bg[h]);
     }
-    const float bg_dot = (f.bg0 * g0 + f.bg1 * g1) + f.bg2 * g2;
-    float Tr = Tf;
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f; // accumulated colour behind the current splat
-    const float fpx = float(px), fpy = float(py);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float fx0 = float(tx * kTile + ox), fx1 = fx0 + float(kSide - 1), fy0 = float(ty * kTile + oy), fy1 = fy0 + float(kSide - 1);
-    for (int32_t hi = max_n; hi > 0; hi -= kThreads) {
-        const int32_t lo = hi > kThreads ? hi - kThreads : 0;
-        __syncthreads();
-        // the batch's records that can reach a pixel of this block (the
+    p.Tr = f2(T[0], T[1]);
+    p.a0 = p.a1 = p.a2 = f2(0.f);
+    p.g0 = f2(g[0][0], g[1][0]);
+    p.g1 = f2(g[0][1], g[1][1]);
+    p.g2 = f2(g[0][2], g[1][2]);
+    p.bg = f2(bg[0], bg[1]);
+    p.n0 = n[0];
+    p.n1 = n[1];
+    plain = __all_sync(0xffffffffu, plain);
+    const int32_t b = ranges[2 * tile];
+    const int32_t end = __reduce_max_sync(0xffffffffu, max(n[0], n[1]));
+    const float fpx = float(px);
+    const F2 fpy = f2(float(py), float(py + 4u));
+    const float fx0 = float(x0), fx1 = fx0 + 7.f, fy0 = float(y0), fy1 = fy0 + 7.f;
+    float held[9] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
+    uint32_t held_id = 0xffffffffu;
+    const int my_slot = lane == 1 ? 8 : (((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1));
+    const bool adds = (lane & 3) == 0 || lane == 1;
+    const auto add = [&](double w, double ninth) {
+        // lanes 0, 4, ..., 28 hold slots 0 to 7; lane 1 adds slot 8
+        const double total = lane == 1 ? ninth : w;
+        if (adds && held_id != 0xffffffffu && total != 0.0)
+            atomicAdd(acc + size_t(held_id) * 9 + my_slot, total);
+    };
+    for (int32_t hi = end; hi > 0; hi -= 32) {
+        // the batch's records that can reach a pixel of this quarter (the
         // forward's exact rectangle cull), compacted in list order with their
         // list positions; the others add nothing to any pixel here
-        const int32_t k = lo + int32_t(threadIdx.x);
-        uint32_t id = 0;
-        float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
-        int keep = 0;
+        const int32_t k = (hi > 32 ? hi - 32 : 0) + lane;
+        bool keep = false, fine = true;
+        float4 r0, r1, c;
         if (k < hi) {
-            id = list[b + k];
+            const uint32_t id = list[b + k];
             r0 = rec[2 * size_t(id)];
             r1 = rec[2 * size_t(id) + 1];
             const float qmin = rect_min_q(r0.x, r0.y, r0.z, 0.5f * r1.x, r0.w, fx0, fx1, fy0, fy1);
             keep = !(qmin > r1.z * 1.001f + 0.01f);
+            if (keep) {
+                r1.w = __int_as_float(k);
+                c = make_float4(rgb[3 * size_t(id)], rgb[3 * size_t(id) + 1], rgb[3 * size_t(id) + 2], __uint_as_float(id));
+                fine = bwd_plain(((fabsf(r0.x) + fabsf(r0.y)) + fabsf(r1.x)) + (fabsf(r0.z) + fabsf(r0.w)), kBwdPlainGeometry) && bwd_plain(r1.y)
+                    && bwd_plain((fabsf(c.x) + fabsf(c.y)) + fabsf(c.z));
+            }
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0)
-            s_warp_tot[warp] = __popc(m);
-        __syncthreads();
-        int pos = __popc(m & ((1u << lane) - 1u));
-        int n = 0;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const int t = s_warp_tot[w];
-            pos += (w < warp) ? t : 0;
-            n += t;
-        }
+        const bool guarded = !plain || !__all_sync(0xffffffffu, fine);
+        __syncwarp(); // the last batch is read
         if (keep) {
-            r1.w = __int_as_float(k);
-            s_id[pos] = id;
-            s_r0[pos] = r0;
-            s_r1[pos] = r1;
-            s_rgb[0][pos] = rgb[3 * size_t(id)];
-            s_rgb[1][pos] = rgb[3 * size_t(id) + 1];
-            s_rgb[2][pos] = rgb[3 * size_t(id) + 2];
+            const int pos = __popc(m & ((1u << lane) - 1u));
+            s_r0[warp][pos] = r0;
+            s_r1[warp][pos] = r1;
+            s_rgb[warp][pos] = c;
         }
-        __syncthreads();
-        for (int j = n - 1; j >= 0; --j) {
-            float v[9] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
-            bool any = false;
-            const float4 r0 = s_r0[j], r1 = s_r1[j];
-            const int32_t kk = __float_as_int(r1.w);
-            float dx, dy;
-            const float q = splat_q(r0, r1.x, fpx, fpy, &dx, &dy);
+        __syncwarp();
+        for (int j = __popc(m) - 1; j >= 0; --j) {
+            const float4 q0 = s_r0[warp][j], q1 = s_r1[warp][j];
+            const int32_t kk = __float_as_int(q1.w);
+            // splat_q on both pixels
+            const float dx = fpx - q0.x;
+            const F2 dy = add2(fpy, f2(-q0.y));
+            const F2 q = fma2(fma2(f2(q0.z), f2(dx), mul2(f2(q1.x), dy)), f2(dx), mul2(mul2(f2(q0.w), dy), dy));
+            float qa, qb;
+            split2(q, &qa, &qb);
             // the forward's cutoff: past q_cut alpha < 1/255, so exp is not
             // needed; a record no lane of the warp needs costs one vote
-            const bool need = kk < my_n && !(q > r1.z);
-            if (!__any_sync(0xffffffffu, need))
+            const bool u0 = kk < p.n0 && !(qa > q1.z), u1 = kk < p.n1 && !(qb > q1.z);
+            if (!__any_sync(0xffffffffu, u0 || u1))
                 continue;
-            if (need) {
-                const float4 co = make_float4(r0.z, 0.5f * r1.x, r0.w, r1.y); // conic a, b, c and opacity
-                const float g = dgmr_fm::exp_f_nonpos(-0.5f * q);
-                const float alpha = min_f(0.99f, co.w * g);
-                if (!(alpha < 1.0f / 255.0f)) {
-                    any = true;
-                    // T before this splat, and the background term's 1 / (1 - alpha): one reciprocal
-                    const float inv = 1.f / (1.f - alpha);
-                    Tr = Tr * inv;
-                    const float c0 = s_rgb[0][j], c1 = s_rgb[1][j], c2 = s_rgb[2][j];
-                    const float aT = alpha * Tr;
-                    v[6] = aT * g0;
-                    v[7] = aT * g1;
-                    v[8] = aT * g2;
-                    const float g_alpha = Tr * (((c0 - a0) * g0 + (c1 - a1) * g1) + (c2 - a2) * g2) - (Tf * bg_dot) * inv;
-                    a0 = alpha * c0 + (1.f - alpha) * a0;
-                    a1 = alpha * c1 + (1.f - alpha) * a1;
-                    a2 = alpha * c2 + (1.f - alpha) * a2;
-                    if (co.w * g < 0.99f) {
-                        v[5] = g_alpha * g;
-                        const float g_q = -0.5f * g * (g_alpha * co.w);
-                        v[2] = g_q * dx * dx;
-                        v[3] = g_q * 2.f * dx * dy;
-                        v[4] = g_q * dy * dy;
-                        v[0] = -(g_q * (2.f * co.x * dx + 2.f * co.y * dy));
-                        v[1] = -(g_q * (2.f * co.z * dy + 2.f * co.y * dx));
-                    }
-                }
+            const float4 col = s_rgb[warp][j];
+            // the last record's reduction is issued with this record's body: they
+            // are independent, and each is a long dependent chain
+            float v[9];
+            bool any;
+            double ninth, w;
+            if (guarded) {
+                any = bwd_record<true>(p, q0, q1, col, q, dx, dy, u0, u1, v);
+                w = warp_reduce_scatter9(held, lane, &ninth);
+            } else {
+                any = bwd_record<false>(p, q0, q1, col, q, dx, dy, u0, u1, v);
+                w = warp_reduce_scatter9(held, lane, &ninth);
             }
-            if (__any_sync(0xffffffffu, any)) {
-                // reduce-scatter of the 9 partials over the warp (16 shuffles, not
-                // 9 x 5): lane l ends with the warp's sum of partial slot(l) and
-                // the lanes of slots 0..8 add them, one atomic each.  The totals
-                // over warps are double: in float, the order in which the
-                // atomics of many cancelling terms land moved single elements by
-                // ~1e-3 relative from run to run at 200k Gaussians, 1024^2.
-                float w = warp_reduce_scatter9(v, lane);
-                const int slot = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
-                if ((lane & 1) == 0 && slot < 9 && w != 0.f)
-                    atomicAdd(acc + size_t(s_id[j]) * 9 + slot, double(w));
-            }
+            add(w, ninth);
+            any = __any_sync(0xffffffffu, any);
+            held_id = any ? __float_as_uint(col.w) : 0xffffffffu;
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+                held[k] = v[k];
         }
     }
+    double ninth;
+    const double w = warp_reduce_scatter9(held, lane, &ninth);
+    add(w, ninth);
 }
 
-// The per-pixel adjoint over n_tiles tiles with the forward's block shape.
+// The per-pixel adjoint over n_tiles tiles.
 template <class Frames>
-void launch_blend_bwd(int side, uint32_t n_tiles, const int32_t* ranges, const uint32_t* list, const float4* rec, const float* rgb, double* acc,
+void launch_blend_bwd(uint32_t n_tiles, const int32_t* ranges, const uint32_t* list, const float4* rec, const float* rgb, double* acc,
     const uint32_t* tile_order, const Frames& frames, cudaStream_t s)
 {
     if (n_tiles == 0)
         return;
-    if (side == 8)
-        k_splat_bwd_pixels<8, Frames><<<n_tiles * BlendShape<8>::kPerTile, BlendShape<8>::kThreads, 0, s>>>(ranges, list, rec, rgb, acc, tile_order, frames);
-    else
-        k_splat_bwd_pixels<16, Frames><<<n_tiles, BlendShape<16>::kThreads, 0, s>>>(ranges, list, rec, rgb, acc, tile_order, frames);
+    k_splat_bwd_pixels<Frames><<<n_tiles, kBwdWarps * 32, 0, s>>>(ranges, list, rec, rgb, acc, tile_order, frames);
 }
 
 struct SplatBwdGauss {
@@ -658,16 +775,20 @@ __device__ __forceinline__ void bwd_gaussian_one(const SplatBwdGauss& p, const C
 {
     if (p.tiles_touched[o] == 0)
         return;
-    float a[9];
+    double m[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k)
-        a[k] = float(p.acc[size_t(o) * 9 + k]);
+        m[k] = p.acc[size_t(o) * 9 + k];
     const V3<float> mu = { p.centroids[3 * i], p.centroids[3 * i + 1], p.centroids[3 * i + 2] };
     const V3<float> sc = mul3(V3<float> { p.scales[3 * i], p.scales[3 * i + 1], p.scales[3 * i + 2] }, cam.cov_scale_multiplier);
     const float* q = p.rotations + 4 * size_t(i);
     const M3<float> R = quat_to_mat3(q[0], q[1], q[2], q[3]);
     const Gaussian2d<float> g2 = splat_project(p.form, p.weights[i], mu, sc, R, cam, 0.3f);
     const S2<float> M = inverse2(g2.cov);
+    // q = a dx^2 + 2b dx dy + c dy^2 with d = pixel - centre: the gradients of the
+    // centre and of the conic from the moments of d/dq
+    const float a[9] = { float(-2.0 * (double(M.v[0]) * m[0] + double(M.v[1]) * m[1])), float(-2.0 * (double(M.v[1]) * m[0] + double(M.v[2]) * m[1])),
+        float(m[2]), float(2.0 * m[3]), float(m[4]), float(m[5]), float(m[6]), float(m[7]), float(m[8]) };
     const float G00 = a[2], G01 = a[3] * 0.5f, G11 = a[4];
     // H = -M G M (2x2 symmetric)
     const float MG00 = M.v[0] * G00 + M.v[1] * G01, MG01 = M.v[0] * G01 + M.v[1] * G11;
@@ -1073,7 +1194,7 @@ dgmr_status dgmr_splat_backward(const dgmr_scene* scene, const dgmr_camera* came
     const CameraT<float> cam = make_camera<float>(*camera);
     const int par = tile_sort_parity(super_count(cam.gx, cam.gy));
     cudaMemsetAsync(L.grad_acc, 0, size_t(N) * 9 * sizeof(double), s);
-    launch_blend_bwd(kBlendSide, cam.gx * cam.gy, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, L.grad_acc, L.tile_order,
+    launch_blend_bwd(cam.gx * cam.gy, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, L.grad_acc, L.tile_order,
         single_frame(cam, nullptr, L, grad_framebuffer), s);
     SplatBwdGauss p { N, static_cast<const float*>(scene->centroids), static_cast<const float*>(scene->sh), scene->sh_stride, scene->sh_degree,
         static_cast<const float*>(scene->weights), static_cast<const float*>(scene->scales), static_cast<const float*>(scene->rotations), L.clamped,
@@ -1296,7 +1417,7 @@ dgmr_status dgmr_splat_batch_backward(const dgmr_scene* scenes, int32_t n_scenes
         return DGMR_OK;
     const int par = tile_sort_parity(plan.tab.n_stiles);
     cudaMemsetAsync(L.grad_acc, 0, size_t(G) * 9 * sizeof(double), s);
-    launch_blend_bwd(plan.blend_side, plan.tab.n_tiles, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, L.grad_acc, L.tile_order, plan.tab, s);
+    launch_blend_bwd(plan.tab.n_tiles, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, L.grad_acc, L.tile_order, plan.tab, s);
     SplatBwdGauss state { 0, nullptr, nullptr, 1, 0, nullptr, nullptr, nullptr, L.clamped, L.tiles_touched, L.grad_acc, nullptr, nullptr, nullptr, nullptr,
         nullptr, Formulation::Ots };
     k_batch_bwd_gaussians<<<(n_scene_gaussians + 127) / 128, 128, 0, s>>>(state, plan.tab);
