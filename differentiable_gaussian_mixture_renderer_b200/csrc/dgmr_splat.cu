@@ -29,7 +29,7 @@ struct SplatLayout {
     int32_t* ranges;
     float* final_T;
     int32_t* n_contrib;
-    double* grad_acc; // [N,9]: moments of d/dq (dx, dy, dx^2, dx dy, dy^2), opacity, rgb(3), summed over pixels in double
+    double* grad_acc; // [N,9]: d/dq times (dx, dy, dx^2, 2 dx dy, dy^2), opacity, rgb(3), summed over pixels in double
     float4* blend_rec; // [N,2]: (x, y, a, c), (2b, opacity, q_cut, 0) -- the blend's 32-byte record
     uint32_t* tile_order; // [tiles] launch order of the per-tile kernels, heaviest first
     uint32_t* tile_cost; // [tiles] predicted blend cost of each tile as a bucket, 0 = heaviest
@@ -420,39 +420,32 @@ void launch_blend(int side, uint32_t n_tiles, const int32_t* ranges, const uint3
     note_launch();
 }
 
-// Sums of 9 per-lane values over a warp, scattered.  Slots 0..7: halve the
-// slots each lane holds at every butterfly level (8 -> 4 -> 2 -> 1, the upper half
-// kept by the lanes whose level bit is set), then add the partners left; slot 8: a
-// plain butterfly.  Lane l returns the warp total of slot 4 b4 + 2 b3 + b2 (b =
-// the bits of l) and, in `ninth`, that of slot 8.  The last two levels add in
-// double: the terms of a long thin splat cancel, and a float sum ends at 8 lanes
-// (16 pixels).
-__device__ __forceinline__ double warp_reduce_scatter9(const float (&v)[9], int lane, double* ninth)
+// Sums of 12 per-lane values over a warp, scattered: halve the slots each lane
+// holds at every butterfly level (12 -> 6 -> 3, the upper half kept by the lanes
+// whose level bit is set), exchange one pair of the three and sum the third,
+// then halve the two that are left.  Every sum is the tree over lane distances 16,
+// 8, 4, 2, 1.  Lane l returns the warp total of slot reduce_slot(l), lanes
+// that differ in bit 0 the same one.
+__device__ __forceinline__ int reduce_slot(int lane)
 {
-    float a[8], last = v[8];
+    const int base = 6 * ((lane >> 4) & 1) + 3 * ((lane >> 3) & 1);
+    return base + ((lane & 2) ? 2 : ((lane >> 2) & 1));
+}
+__device__ __forceinline__ float warp_reduce_scatter12(const float (&v)[12], int lane)
+{
+    float a[6], b[3];
+    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0, b1 = (lane & 2) != 0;
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-        a[q] = v[q];
+    for (int q = 0; q < 6; ++q)
+        a[q] = (b4 ? v[q + 6] : v[q]) + __shfl_xor_sync(0xffffffffu, b4 ? v[q] : v[q + 6], 16);
 #pragma unroll
-    for (int half = 4; half >= 1; half >>= 1) {
-        const int bit = half * 4; // the xor distance: 16, 8, 4
-        const bool upper = (lane & bit) != 0;
-#pragma unroll
-        for (int q = 0; q < half; ++q) {
-            const float give = upper ? a[q] : a[q + half];
-            const float keep = upper ? a[q + half] : a[q];
-            a[q] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
-        }
-        last += __shfl_xor_sync(0xffffffffu, last, bit);
-    }
-    double sum = double(a[0]), end = double(last);
-#pragma unroll
-    for (int bit = 2; bit >= 1; bit >>= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, bit);
-        end += __shfl_xor_sync(0xffffffffu, end, bit);
-    }
-    *ninth = end;
-    return sum;
+    for (int q = 0; q < 3; ++q)
+        b[q] = (b3 ? a[q + 3] : a[q]) + __shfl_xor_sync(0xffffffffu, b3 ? a[q] : a[q + 3], 8);
+    // slots 0 and 1 of the three between the lanes of bit 2; slot 2 on both
+    const float c = (b2 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, b2 ? b[0] : b[1], 4);
+    const float d = b[2] + __shfl_xor_sync(0xffffffffu, b[2], 4);
+    const float e = (b1 ? d : c) + __shfl_xor_sync(0xffffffffu, b1 ? c : d, 2);
+    return e + __shfl_xor_sync(0xffffffffu, e, 1);
 }
 
 // Reverse-order blend adjoint.  A warp owns an 8x8 quarter of a tile and a lane
@@ -461,10 +454,12 @@ __device__ __forceinline__ double warp_reduce_scatter9(const float (&v)[9], int 
 // packed operation for both, and a record's partials are summed over 64 pixels
 // by one warp reduction.  Each pixel walks its contributors back to front,
 // recovering T_i = T_{i+1} / (1 - alpha_i).  Per record the warp sums the
-// moments of g_q = d/dq over its pixels (g_q dx, g_q dy, g_q dx^2, g_q dx dy,
-// g_q dy^2), d/dopacity and d/drgb -- the centre's and the conic's gradients are
-// linear in the moments, which k_splat_bwd_gaussians applies to the totals -- and
-// nine lanes add one value each.  The totals over warps are double: in float,
+// moments of g_q = d/dq over its pixels (g_q dx and g_q dy, from which
+// k_splat_bwd_gaussians takes the centre's gradient), the conic's gradients (g_q
+// dx^2, 2 g_q dx dy, g_q dy^2), d/dopacity and d/drgb, and twelve lanes add one
+// value each.  The conic's three are summed over 32 pixels at a time, upper and
+// lower half apart: the chain to a long thin splat's scales cancels by 10^5, and
+// with a float sum over 64 pixels single elements moved by 1e-3.  The totals over warps are double: in float,
 // the order in which the atomics of many cancelling terms land moved single
 // elements by ~1e-3 relative from run to run at 200k Gaussians, 1024^2.
 // Tiles run in the forward's launch order (heaviest predicted walk first); a
@@ -473,9 +468,8 @@ __device__ __forceinline__ double warp_reduce_scatter9(const float (&v)[9], int 
 // Bound by instruction issue, and at the end of a launch by the longest warp's
 // serial walk: so a record's reduction is issued with the next record's body, and
 // 80 registers without spills (six blocks per SM) beat 64 with them.  Against a
-// pixel per lane, a reduction per 32 pixels and 48 registers, forward + backward
-// (mean of four cameras): 0.946 -> 0.800 ms at 200k, 1024^2; 1.323 -> 1.192 ms at
-// 1M, 1080p; 6.42 -> 5.47 ms for 12 batched views.
+// pixel per lane, a reduction per 32 pixels of all nine values and 48 registers:
+// 406 -> 327 us at 1M, 1080p; 430 -> 297 us at 200k, 1024^2.
 constexpr int kBwdWarps = 4; // the quarters of a tile
 static_assert(kTile == 16, "four 8x8 quarters per tile");
 
@@ -498,7 +492,7 @@ struct BwdPixels {
 // Returns whether any partial is nonzero.  kGuarded: values may be huge or not
 // finite, and a pixel that does not use the record must not see them.
 template <bool kGuarded>
-__device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, float4 c, F2 q, float dx, F2 dy, bool use0, bool use1, float (&v)[9])
+__device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, float4 c, F2 q, float dx, F2 dy, bool use0, bool use1, float (&v)[12])
 {
     const float op = r1.y;
     float e0, e1;
@@ -524,7 +518,8 @@ __device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, f
     al1 = use1 ? al1 : 0.f;
     const F2 g = f2(use0 ? e0 : 0.f, use1 ? e1 : 0.f), alpha = f2(al0, al1);
     // 1 / (1 - alpha), 1 - alpha in [0.01, 1]: the hardware's approximation and
-    // one Newton step y + y (1 - x y)
+    // one Newton step y + y (1 - x y), the correctly rounded quotient for every
+    // float in [0.0099, 1] (compared once with the division)
     const float x0 = 1.f - al0, x1 = 1.f - al1;
     float y0, y1;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(x0));
@@ -536,41 +531,43 @@ __device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, f
     const F2 w0 = mul2(aT, p.g0), w1 = mul2(aT, p.g1), w2 = mul2(aT, p.g2);
     const F2 neg = f2(-1.f);
     const F2 d0 = fma2(p.a0, neg, f2(c.x)), d1 = fma2(p.a1, neg, f2(c.y)), d2 = fma2(p.a2, neg, f2(c.z));
-    const F2 dot = fma2(d2, p.g2, fma2(d1, p.g1, mul2(d0, p.g0)));
-    const F2 ga = fma2(Tr, dot, mul2(mul2(p.bg, neg), inv));
+    const F2 dot = add2(add2(mul2_rounded(d0, p.g0), mul2_rounded(d1, p.g1)), mul2_rounded(d2, p.g2));
+    const F2 ga = add2(mul2_rounded(Tr, dot), mul2_rounded(mul2(p.bg, neg), inv));
     float ga0, ga1;
     split2(ga, &ga0, &ga1);
     ga0 = og0 < 0.99f ? ga0 : 0.f; // alpha = 0.99 there, whatever the opacity
     ga1 = og1 < 0.99f ? ga1 : 0.f;
     const F2 go = mul2(f2(ga0, ga1), g); // d/dopacity
-    const F2 gq = mul2(go, f2(-0.5f * op));
-    const F2 gy = mul2(gq, dy), gyy = mul2(gy, dy);
-    const F2 na0 = fma2(alpha, d0, p.a0), na1 = fma2(alpha, d1, p.a1), na2 = fma2(alpha, d2, p.a2);
+    const F2 gq = mul2(mul2(g, f2(-0.5f)), mul2(f2(ga0, ga1), f2(op)));
+    const F2 gx = mul2(gq, f2(dx)), gy = mul2(gq, dy);
+    const F2 gxx = mul2(gx, f2(dx)), gxy = mul2(mul2(gx, f2(2.f)), dy), gyy = mul2(gy, dy);
+    const F2 keep = f2(x0, x1); // 1 - alpha
+    const F2 na0 = add2(mul2_rounded(alpha, f2(c.x)), mul2_rounded(keep, p.a0));
+    const F2 na1 = add2(mul2_rounded(alpha, f2(c.y)), mul2_rounded(keep, p.a1));
+    const F2 na2 = add2(mul2_rounded(alpha, f2(c.z)), mul2_rounded(keep, p.a2));
+    const auto halves = [&](F2 t, float* lo, float* hi) {
+        split2(t, lo, hi);
+        if (kGuarded) {
+            *lo = use0 ? *lo : 0.f;
+            *hi = use1 ? *hi : 0.f;
+        }
+    };
     const auto sum = [&](F2 t) {
         float lo, hi;
-        split2(t, &lo, &hi);
-        if (kGuarded) {
-            lo = use0 ? lo : 0.f;
-            hi = use1 ? hi : 0.f;
-        }
+        halves(t, &lo, &hi);
         return lo + hi;
     };
-    const float s = sum(gq);
-    v[0] = dx * s;
+    // in the order of k_splat_bwd_pixels' accumulators
+    v[0] = sum(gx);
     v[1] = sum(gy);
-    v[2] = dx * v[0];
-    v[3] = dx * v[1];
-    v[4] = sum(gyy);
-    v[5] = sum(go);
-    v[6] = sum(w0);
-    v[7] = sum(w1);
-    v[8] = sum(w2);
+    halves(gxx, &v[2], &v[3]);
+    halves(gxy, &v[4], &v[5]);
+    halves(gyy, &v[6], &v[7]);
+    v[8] = sum(go);
+    v[9] = sum(w0);
+    v[10] = sum(w1);
+    v[11] = sum(w2);
     if (kGuarded) {
-        if (!use0 && !use1) {
-#pragma unroll
-            for (int k = 0; k < 9; ++k)
-                v[k] = 0.f; // dx may not be finite
-        }
         const auto pick = [&](F2& to, F2 from) {
             float a, b, x, y;
             split2(to, &a, &b);
@@ -641,15 +638,15 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 6) k_splat_bwd_pixels(const in
     const float fpx = float(px);
     const F2 fpy = f2(float(py), float(py + 4u));
     const float fx0 = float(x0), fx1 = fx0 + 7.f, fy0 = float(y0), fy1 = fy0 + 7.f;
-    float held[9] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
+    float held[12] = {};
     uint32_t held_id = 0xffffffffu;
-    const int my_slot = lane == 1 ? 8 : (((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1));
-    const bool adds = (lane & 3) == 0 || lane == 1;
-    const auto add = [&](double w, double ninth) {
-        // lanes 0, 4, ..., 28 hold slots 0 to 7; lane 1 adds slot 8
-        const double total = lane == 1 ? ninth : w;
-        if (adds && held_id != 0xffffffffu && total != 0.0)
-            atomicAdd(acc + size_t(held_id) * 9 + my_slot, total);
+    // the accumulator of each reduced slot: 0, 1, then the conic's three from both halves, then opacity and colour
+    const int slot = reduce_slot(lane);
+    const int my_slot = slot < 2 ? slot : slot < 8 ? 1 + slot / 2 : slot - 3;
+    const bool adds = (lane & 1) == 0 && ((lane & 2) == 0 || (lane & 4) == 0); // slot 2 of three is on both lanes of bit 2
+    const auto add = [&](float total) {
+        if (adds && held_id != 0xffffffffu && total != 0.f)
+            atomicAdd(acc + size_t(held_id) * 9 + my_slot, double(total));
     };
     for (int32_t hi = end; hi > 0; hi -= 32) {
         // the batch's records that can reach a pixel of this quarter (the
@@ -698,27 +695,24 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 6) k_splat_bwd_pixels(const in
             const float4 col = s_rgb[warp][j];
             // the last record's reduction is issued with this record's body: they
             // are independent, and each is a long dependent chain
-            float v[9];
+            float v[12], w;
             bool any;
-            double ninth, w;
             if (guarded) {
                 any = bwd_record<true>(p, q0, q1, col, q, dx, dy, u0, u1, v);
-                w = warp_reduce_scatter9(held, lane, &ninth);
+                w = warp_reduce_scatter12(held, lane);
             } else {
                 any = bwd_record<false>(p, q0, q1, col, q, dx, dy, u0, u1, v);
-                w = warp_reduce_scatter9(held, lane, &ninth);
+                w = warp_reduce_scatter12(held, lane);
             }
-            add(w, ninth);
+            add(w);
             any = __any_sync(0xffffffffu, any);
             held_id = any ? __float_as_uint(col.w) : 0xffffffffu;
 #pragma unroll
-            for (int k = 0; k < 9; ++k)
+            for (int k = 0; k < 12; ++k)
                 held[k] = v[k];
         }
     }
-    double ninth;
-    const double w = warp_reduce_scatter9(held, lane, &ninth);
-    add(w, ninth);
+    add(warp_reduce_scatter12(held, lane));
 }
 
 // The per-pixel adjoint over n_tiles tiles.
@@ -782,8 +776,8 @@ __device__ __forceinline__ void zero_sh_grads(const SplatBwdGauss& p, uint32_t i
 // result is added to `sum` and, for the SH coefficients, written to their
 // gradient rows (kAddSh: added to them), so several views of one scene sum up.
 // Rows and sums are stored once per Gaussian (zeroed first and added to in
-// memory: 106.6 us at 1M, SH degree 0, now 85.4; bound by its ~1700 instructions
-// per warp, 29 us of memory traffic).
+// memory, with the same arithmetic: 106.6 us at 1M, SH degree 0, now 85.9; bound by
+// its ~1700 instructions per warp, 29 us of memory traffic).
 template <bool kAddSh>
 __device__ __forceinline__ void bwd_gaussian_one(const SplatBwdGauss& p, const CameraT<float>& cam, uint32_t i, uint32_t o, GaussianGrads& sum)
 {
@@ -797,10 +791,10 @@ __device__ __forceinline__ void bwd_gaussian_one(const SplatBwdGauss& p, const C
     const M3<float> R = quat_to_mat3(q[0], q[1], q[2], q[3]);
     const Gaussian2d<float> g2 = splat_project(p.form, p.weights[i], mu, sc, R, cam, 0.3f);
     const S2<float> M = inverse2(g2.cov);
-    // q = a dx^2 + 2b dx dy + c dy^2 with d = pixel - centre: the gradients of the
-    // centre and of the conic from the moments of d/dq
+    // q = a dx^2 + 2b dx dy + c dy^2 with d = pixel - centre: the centre's
+    // gradient from the moments of d/dq
     const float a[9] = { float(-2.0 * (double(M.v[0]) * m[0] + double(M.v[1]) * m[1])), float(-2.0 * (double(M.v[1]) * m[0] + double(M.v[2]) * m[1])),
-        float(m[2]), float(2.0 * m[3]), float(m[4]), float(m[5]), float(m[6]), float(m[7]), float(m[8]) };
+        float(m[2]), float(m[3]), float(m[4]), float(m[5]), float(m[6]), float(m[7]), float(m[8]) };
     const float G00 = a[2], G01 = a[3] * 0.5f, G11 = a[4];
     // H = -M G M (2x2 symmetric)
     const float MG00 = M.v[0] * G00 + M.v[1] * G01, MG01 = M.v[0] * G01 + M.v[1] * G11;
