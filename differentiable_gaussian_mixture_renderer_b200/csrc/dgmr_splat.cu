@@ -232,6 +232,25 @@ __device__ __forceinline__ float rect_min_q(float cx, float cy, float a, float b
     return m;
 }
 
+// The packed walks (two pixels per lane, the halves of packed floats) take
+// records and pixels of ordinary magnitude: the half that does not use a record is
+// multiplied by an exact zero, which needs finite operands (products of two
+// values up to kPlain are finite), and its exp is evaluated without the tests for
+// special cases.  So the conic has to be positive definite, and close enough to
+// the 8x8 quarter for the rounding of the quadratic form (4 ulp of its terms) to
+// stay far above the -170 where exp(-q/2) overflows, and q_cut (NaN for a negative
+// opacity) to keep it off the range where the exp is subnormal; it bounds the
+// opacity too, by e^50 / 255.  Other records take the guarded walk.
+constexpr float kPlain = 1.0e18f, kPlainForm = 1.0e8f, kPlainCut = 100.f;
+__device__ __forceinline__ bool plain_value(float x) { return fabsf(x) <= kPlain; } // false for NaN
+__device__ __forceinline__ bool plain_record(float4 r0, float4 r1, float4 rgb, float x0, float y0)
+{
+    const float dx = fabsf(r0.x - x0) + 8.f, dy = fabsf(r0.y - y0) + 8.f;
+    const float b = 0.5f * r1.x;
+    return r0.z > 0.f && r0.w > 0.f && r0.z * r0.w - b * b > 0.f && (r0.z + r0.w) * (dx * dx + dy * dy) <= kPlainForm && r1.z <= kPlainCut
+        && plain_value((fabsf(rgb.x) + fabsf(rgb.y)) + fabsf(rgb.z));
+}
+
 // One 16x16 tile per block of 256 threads, one pixel per thread.  Each batch
 // of up to 256 list entries is loaded one per thread; splats whose cutoff
 // ellipse cannot reach the tile are dropped (an exact rectangle minimum with a
@@ -254,29 +273,17 @@ struct SingleFrame {
     __device__ __forceinline__ FrameRef frame(uint32_t tile) const { return FrameRef { W, H, gx, tile, bg0, bg1, bg2, fb, final_T, n_contrib, grad_fb }; }
 };
 
-// Block shapes of the blend: a 16x16 tile per block of 256 threads, or an 8x8
-// quarter of a tile per block of 64 threads (four blocks walk the same tile
-// list, each culling against its own quarter and stopping when its own pixels
-// are saturated; every pixel sees the same records in the same order, so the
-// results are the same bits).  __launch_bounds__ keeps both at 48 registers:
-// for 16x16, five blocks per SM instead of four at the 52 the compiler picks
-// unbounded -- 3 % shorter launches over 8 cameras at 1080p/1M, +2.3 % served
-// renders/s.
-template <int kSide>
-struct BlendShape {
-    static_assert(kSide == 16 || kSide == 8, "blend blocks of 16x16 or 8x8 pixels");
-    static constexpr int kThreads = kSide * kSide;
-    static constexpr int kMinBlocks = kSide == 16 ? 5 : 20;
-    static constexpr int kPerTile = (int(kTile) / kSide) * (int(kTile) / kSide); // blocks per 16x16 tile
-};
-
-template <int kSide, class Frames>
-__global__ void __launch_bounds__(BlendShape<kSide>::kThreads, BlendShape<kSide>::kMinBlocks) k_splat_blend(const int32_t* __restrict__ ranges,
-    const uint32_t* __restrict__ list, const float4* __restrict__ rec, const float* __restrict__ rgb, uint32_t N, uint32_t cap, uint32_t* __restrict__ stats,
+// The blend with a 16x16 tile per block of 256 threads, a pixel each (batches may
+// choose it, dgmr_batch_view.blend_block; the same bits as the quarters below).
+// __launch_bounds__ keeps it at 48 registers, five blocks per SM instead of four at
+// the 52 the compiler picks unbounded: 3 % shorter launches over 8 cameras at
+// 1080p/1M.
+template <class Frames>
+__global__ void __launch_bounds__(kTilePixels, 5) k_splat_blend_tiles(const int32_t* __restrict__ ranges, const uint32_t* __restrict__ list,
+    const float4* __restrict__ rec, const float* __restrict__ rgb, uint32_t N, uint32_t cap, uint32_t* __restrict__ stats,
     const uint32_t* __restrict__ tile_order, const __grid_constant__ Frames frames)
 {
-    constexpr int kThreads = BlendShape<kSide>::kThreads;
-    constexpr int kPerTile = BlendShape<kSide>::kPerTile;
+    constexpr int kThreads = kTilePixels;
     constexpr int kBatch = kThreads;
     constexpr int kWarps = kThreads / 32;
     constexpr int kGroup = 4;
@@ -285,20 +292,16 @@ __global__ void __launch_bounds__(BlendShape<kSide>::kThreads, BlendShape<kSide>
     __shared__ float4 s_r1[kBatch]; // (2b, opacity, q_cut, 1-based list index as int bits)
     __shared__ float4 s_rgb[kBatch]; // (r, g, b, .): one 16-byte load per record that a warp blends
     __shared__ int s_warp_tot[kWarps];
-    const unsigned slot = blockIdx.x / kPerTile, part = blockIdx.x % kPerTile;
-    const unsigned tile = tile_order ? tile_order[slot] : slot;
+    const unsigned tile = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
     const FrameRef f = frames.frame(tile);
     const unsigned W = f.W, H = f.H;
     const unsigned tx = f.tile % f.gx, ty = f.tile / f.gx;
-    // the block's pixels start at (ox, oy) of the tile; warp w covers the 8x4
-    // pixel block (8 (w % kRow), 4 (w / kRow)) of them: a compact footprint, so
-    // fewer records pass some lane's cutoff than over a 16x2 strip (a record
-    // no lane needs costs one vote)
-    constexpr unsigned kRow = unsigned(kSide) / 8u;
-    const unsigned ox = unsigned(kSide) * (part % (kTile / unsigned(kSide))), oy = unsigned(kSide) * (part / (kTile / unsigned(kSide)));
+    // warp w covers the 8x4 pixel block (8 (w % 2), 4 (w / 2)) of the tile: a
+    // compact footprint, so fewer records pass some lane's cutoff than over a 16x2
+    // strip (a record no lane needs costs one vote)
     const unsigned wb = threadIdx.x >> 5;
-    const unsigned px = tx * kTile + ox + 8u * (wb % kRow) + (threadIdx.x & 7u);
-    const unsigned py = ty * kTile + oy + 4u * (wb / kRow) + ((threadIdx.x >> 3) & 3u);
+    const unsigned px = tx * kTile + 8u * (wb & 1u) + (threadIdx.x & 7u);
+    const unsigned py = ty * kTile + 4u * (wb >> 1) + ((threadIdx.x >> 3) & 3u);
     PixelState p0 { 1.f, 0.f, 0.f, 0.f, 0, !(px < W && py < H) };
     const bool in0 = !p0.done;
     int32_t b = ranges[2 * tile], e = ranges[2 * tile + 1];
@@ -307,7 +310,7 @@ __global__ void __launch_bounds__(BlendShape<kSide>::kThreads, BlendShape<kSide>
             flag_bounds(stats, 0x31u);
         b = e = 0;
     }
-    const float fx0 = float(tx * kTile + ox), fx1 = fx0 + float(kSide - 1), fy0 = float(ty * kTile + oy), fy1 = fy0 + float(kSide - 1);
+    const float fx0 = float(tx * kTile), fx1 = fx0 + float(kTile - 1), fy0 = float(ty * kTile), fy1 = fy0 + float(kTile - 1);
     const float fpx = float(px), fpy = float(py);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int32_t base = b; base < e; base += kBatch) {
@@ -402,10 +405,228 @@ __global__ void __launch_bounds__(BlendShape<kSide>::kThreads, BlendShape<kSide>
     }
 }
 
-// The blend over n_tiles tiles with blocks of side x side pixels (16 or 8).
-// Single frames use 8x8 blocks: at 1080p with 1M Gaussians the blend takes
-// 0.1725 ms against 0.198 ms with 16x16 blocks (the same bits); batches take
-// the side from their views (dgmr_batch_view.blend_block).
+// The blend with a warp per 8x8 quarter of a tile and two pixels per lane, (x, y)
+// and (x, y + 4), as the halves of packed floats: one packed operation evaluates
+// a record for both, bit for bit what a pixel per thread gives.  The quarters of
+// a tile are independent warps -- each culls the tile's list against its own
+// pixels, 32 entries at a time, and stops when they are saturated -- so there is
+// no block barrier.  A launch ends with its slowest warp's serial walk (some 2000
+// records), so the walk's latencies are overlapped rather than its instructions
+// saved: the next batch is requested ahead (ListWalk: 226 -> 177 us at 1M, 1080p
+// for a camera with a few slow tiles), a group's four exps are evaluated together,
+// needed or not, and 92 registers without spills beat more warps (177 -> 133).
+constexpr int kQuarterWarps = 4;
+// A warp's walk of a tile's list, 32 entries at a time: the next batch's records
+// and the ids of the one after are requested before the current batch is
+// worked on.  (Loaded when their batch began, list, record and colour were three
+// latencies in a row, 94 times for the 3000 entries of a slow tile, and the
+// launch waits for its slowest tile.)
+struct ListWalk {
+    float4 r0, r1; // of the lane's entry in the next batch
+    float c0, c1, c2;
+    uint32_t id, later; // its Gaussian, and that of the batch after
+    __device__ __forceinline__ static uint32_t entry(const uint32_t* __restrict__ list, int32_t k, int32_t first, int32_t end)
+    {
+        return k >= first && k < end ? list[k] : 0xffffffffu;
+    }
+    __device__ __forceinline__ void request(const float4* __restrict__ rec, const float* __restrict__ rgb, uint32_t N)
+    {
+        const size_t g = id < N ? id : 0u;
+        r0 = rec[2 * g];
+        r1 = rec[2 * g + 1];
+        c0 = rgb[3 * g];
+        c1 = rgb[3 * g + 1];
+        c2 = rgb[3 * g + 2];
+    }
+};
+
+struct QuarterPixels {
+    F2 T, c0, c1, c2;
+    int32_t last0, last1;
+    bool done0, done1;
+};
+
+template <bool kGuarded>
+__device__ __forceinline__ void blend_record2(QuarterPixels& p, F2 q, F2 ex, bool use0, bool use1, float4 r1, float4 c)
+{
+    float e0, e1;
+    split2(ex, &e0, &e1);
+    if (kGuarded) {
+        float q0, q1;
+        split2(q, &q0, &q1);
+        if (use0 && !(q0 >= -170.f && q0 <= 170.f))
+            e0 = dgmr_fm::exp_f_nonpos(-0.5f * q0);
+        if (use1 && !(q1 >= -170.f && q1 <= 170.f))
+            e1 = dgmr_fm::exp_f_nonpos(-0.5f * q1);
+    }
+    const float a0 = min_f(0.99f, r1.y * e0), a1 = min_f(0.99f, r1.y * e1);
+    const F2 alpha = f2(a0, a1);
+    const F2 test = mul2(p.T, fma2(alpha, f2(-1.f), f2(1.f)));
+    float t0, t1, T0, T1, w0, w1;
+    split2(test, &t0, &t1);
+    split2(p.T, &T0, &T1);
+    split2(mul2(alpha, p.T), &w0, &w1);
+    const bool live0 = use0 && !(a0 < 1.0f / 255.0f), live1 = use1 && !(a1 < 1.0f / 255.0f);
+    const bool stop0 = live0 && t0 < 0.0001f, stop1 = live1 && t1 < 0.0001f;
+    const bool take0 = live0 && !stop0, take1 = live1 && !stop1;
+    if (kGuarded) {
+        const auto add = [&](F2& to, float col) {
+            float lo, hi;
+            split2(to, &lo, &hi);
+            to = f2(take0 ? __fmaf_rn(col, w0, lo) : lo, take1 ? __fmaf_rn(col, w1, hi) : hi);
+        };
+        add(p.c0, c.x);
+        add(p.c1, c.y);
+        add(p.c2, c.z);
+    } else {
+        const F2 w = f2(take0 ? w0 : 0.f, take1 ? w1 : 0.f);
+        p.c0 = fma2(f2(c.x), w, p.c0);
+        p.c1 = fma2(f2(c.y), w, p.c1);
+        p.c2 = fma2(f2(c.z), w, p.c2);
+    }
+    p.T = f2(take0 ? t0 : T0, take1 ? t1 : T1);
+    const int32_t idx = __float_as_int(r1.w);
+    p.last0 = take0 ? idx : p.last0;
+    p.last1 = take1 ? idx : p.last1;
+    p.done0 = p.done0 || stop0;
+    p.done1 = p.done1 || stop1;
+}
+
+template <class Frames>
+__global__ void __launch_bounds__(kQuarterWarps * 32, 5) k_splat_blend_quarters(const int32_t* __restrict__ ranges, const uint32_t* __restrict__ list,
+    const float4* __restrict__ rec, const float* __restrict__ rgb, uint32_t N, uint32_t cap, uint32_t* __restrict__ stats,
+    const uint32_t* __restrict__ tile_order, const __grid_constant__ Frames frames)
+{
+    constexpr int kGroup = 4;
+    __shared__ float4 s_r0[kQuarterWarps][32];
+    __shared__ float4 s_r1[kQuarterWarps][32]; // (2b, opacity, q_cut, 1-based list index as int bits)
+    __shared__ float4 s_rgb[kQuarterWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned tile = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
+    const FrameRef f = frames.frame(tile);
+    const unsigned W = f.W, H = f.H;
+    const unsigned x0 = (f.tile % f.gx) * kTile + 8u * (unsigned(warp) & 1u), y0 = (f.tile / f.gx) * kTile + 8u * (unsigned(warp) >> 1);
+    const unsigned px = x0 + (unsigned(lane) & 7u), py = y0 + (unsigned(lane) >> 3);
+    const bool in0 = px < W && py < H, in1 = px < W && py + 4u < H;
+    QuarterPixels p { f2(1.f), f2(0.f), f2(0.f), f2(0.f), 0, 0, !in0, !in1 };
+    int32_t b = ranges[2 * tile], e = ranges[2 * tile + 1];
+    if (b < 0 || e < b || uint32_t(e) > cap) {
+        if (threadIdx.x == 0)
+            flag_bounds(stats, 0x31u);
+        b = e = 0;
+    }
+    const float fpx = float(px), fx0 = float(x0), fx1 = fx0 + 7.f, fy0 = float(y0), fy1 = fy0 + 7.f;
+    const F2 fpy = f2(float(py), float(py + 4u));
+    using Walk = ListWalk;
+    Walk next;
+    next.id = Walk::entry(list, b + lane, b, e);
+    next.later = Walk::entry(list, b + 32 + lane, b, e);
+    next.request(rec, rgb, N);
+    for (int32_t base = b; base < e; base += 32) {
+        if (__all_sync(0xffffffffu, p.done0 && p.done1))
+            break;
+        const int32_t k = base + lane;
+        bool keep = false, fine = true;
+        const float4 r0 = next.r0;
+        float4 r1 = next.r1;
+        const float4 c = make_float4(next.c0, next.c1, next.c2, 0.f);
+        const uint32_t g = next.id;
+        next.id = next.later;
+        next.later = Walk::entry(list, k + 64, b, e);
+        next.request(rec, rgb, N);
+        if (k < e) {
+            if (g >= N)
+                flag_bounds(stats, 0x32u);
+            const float qmin = rect_min_q(r0.x, r0.y, r0.z, 0.5f * r1.x, r0.w, fx0, fx1, fy0, fy1);
+            keep = !(qmin > r1.z * 1.001f + 0.01f);
+            if (keep) {
+                r1.w = __int_as_float(k - b + 1);
+                fine = plain_record(r0, r1, c, fx0, fy0);
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        const bool guarded = !__all_sync(0xffffffffu, fine);
+        const int n = __popc(m);
+        __syncwarp(); // the last batch is read
+        if (keep) {
+            const int pos = __popc(m & ((1u << lane) - 1u));
+            s_r0[warp][pos] = r0;
+            s_r1[warp][pos] = r1;
+            s_rgb[warp][pos] = c;
+        }
+        // up to the group boundary: a cutoff below every quadratic form (q = 0
+        // here), so no lane ever uses them
+        if (lane < kGroup - 1 && n + lane < 32) {
+            s_r0[warp][n + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+            s_r1[warp][n + lane] = make_float4(0.f, 0.f, -1.f, 0.f);
+            s_rgb[warp][n + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncwarp();
+        // kGroup records at a time: their quadratic forms (independent), then, in
+        // list order, the exp and the blend step of each record that some
+        // lane's cutoff admits
+        for (int j = 0; j < n; j += kGroup) {
+            F2 q[kGroup];
+            bool u0[kGroup], u1[kGroup];
+#pragma unroll
+            for (int i = 0; i < kGroup; ++i) {
+                const float4 s0 = s_r0[warp][j + i], s1 = s_r1[warp][j + i]; // j + i < 32
+                const float dx = fpx - s0.x;
+                const F2 dy = add2(fpy, f2(-s0.y));
+                q[i] = fma2(fma2(f2(s0.z), f2(dx), mul2(f2(s1.x), dy)), f2(dx), mul2(mul2(f2(s0.w), dy), dy));
+                float qa, qb;
+                split2(q[i], &qa, &qb);
+                u0[i] = !(qa > s1.z);
+                u1[i] = !(qb > s1.z);
+            }
+            bool any = false;
+#pragma unroll
+            for (int i = 0; i < kGroup; ++i) {
+                u0[i] = u0[i] && !p.done0;
+                u1[i] = u1[i] && !p.done1;
+                any = any || u0[i] || u1[i];
+            }
+            if (!__any_sync(0xffffffffu, any))
+                continue;
+            F2 ex[kGroup];
+#pragma unroll
+            for (int i = 0; i < kGroup; ++i)
+                ex[i] = exp2_nonpos(mul2(q[i], f2(-0.5f)));
+            if (guarded) {
+#pragma unroll
+                for (int i = 0; i < kGroup; ++i)
+                    blend_record2<true>(p, q[i], ex[i], u0[i] && !p.done0, u1[i] && !p.done1, s_r1[warp][j + i], s_rgb[warp][j + i]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < kGroup; ++i)
+                    blend_record2<false>(p, q[i], ex[i], u0[i] && !p.done0, u1[i] && !p.done1, s_r1[warp][j + i], s_rgb[warp][j + i]);
+            }
+            if (__all_sync(0xffffffffu, p.done0 && p.done1))
+                break;
+        }
+    }
+    const size_t plane = size_t(W) * H;
+    float T[2], col[3][2];
+    split2(p.T, &T[0], &T[1]);
+    split2(p.c0, &col[0][0], &col[0][1]);
+    split2(p.c1, &col[1][0], &col[1][1]);
+    split2(p.c2, &col[2][0], &col[2][1]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        if (h ? in1 : in0) {
+            const size_t pix = size_t(py + 4u * unsigned(h)) * W + px;
+            f.fb[pix] = col[0][h] + T[h] * f.bg0;
+            f.fb[plane + pix] = col[1][h] + T[h] * f.bg1;
+            f.fb[2 * plane + pix] = col[2][h] + T[h] * f.bg2;
+            f.final_T[pix] = T[h];
+            f.n_contrib[pix] = h ? p.last1 : p.last0;
+        }
+}
+
+// The blend over n_tiles tiles: a warp per 8x8 quarter (side 8), or a block per
+// tile (16).  Single frames use quarters, 157 -> 133 us at 1M, 1080p and 148 -> 135
+// at 200k, 1024^2 against a pixel per thread; batches take the side from their
+// views (dgmr_batch_view.blend_block).
 constexpr int kBlendSide = 8;
 template <class Frames>
 void launch_blend(int side, uint32_t n_tiles, const int32_t* ranges, const uint32_t* list, const float4* rec, const float* rgb, uint32_t N, uint32_t cap,
@@ -414,9 +635,9 @@ void launch_blend(int side, uint32_t n_tiles, const int32_t* ranges, const uint3
     if (n_tiles == 0)
         return;
     if (side == 8)
-        k_splat_blend<8, Frames><<<n_tiles * BlendShape<8>::kPerTile, BlendShape<8>::kThreads, 0, s>>>(ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
+        k_splat_blend_quarters<Frames><<<n_tiles, kQuarterWarps * 32, 0, s>>>(ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
     else
-        k_splat_blend<16, Frames><<<n_tiles, BlendShape<16>::kThreads, 0, s>>>(ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
+        k_splat_blend_tiles<Frames><<<n_tiles, kTilePixels, 0, s>>>(ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
     note_launch();
 }
 
@@ -467,18 +688,12 @@ __device__ __forceinline__ float warp_reduce_scatter12(const float (&v)[12], int
 //
 // Bound by instruction issue, and at the end of a launch by the longest warp's
 // serial walk: so a record's reduction is issued with the next record's body, and
-// 80 registers without spills (six blocks per SM) beat 64 with them.  Against a
+// 80 registers without spills beat 64 with them, and the next batch is requested
+// ahead (ListWalk: 299 -> 273 us at 1M, 1080p, 284 -> 288 at 200k, 1024^2).  Against a
 // pixel per lane, a reduction per 32 pixels of all nine values and 48 registers:
-// 406 -> 327 us at 1M, 1080p; 430 -> 297 us at 200k, 1024^2.
+// 406 -> 273 us at 1M, 1080p; 430 -> 288 us at 200k, 1024^2.
 constexpr int kBwdWarps = 4; // the quarters of a tile
 static_assert(kTile == 16, "four 8x8 quarters per tile");
-
-// The largest magnitude that the packed walk takes from a record or a pixel: the
-// half that does not use a record is multiplied by an exact zero, which needs
-// finite operands (products of two such values are finite, and so is the
-// quadratic form of such a geometry).  Others take the guarded walk.
-constexpr float kBwdPlain = 1.0e18f, kBwdPlainGeometry = 1.0e9f;
-__device__ __forceinline__ bool bwd_plain(float x, float most = kBwdPlain) { return fabsf(x) <= most; } // false for NaN
 
 struct BwdPixels {
     F2 Tr; // transmittance in front of the records walked so far
@@ -497,18 +712,13 @@ __device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, f
     const float op = r1.y;
     float e0, e1;
     split2(exp2_nonpos(mul2(q, f2(-0.5f))), &e0, &e1);
-    {
+    if (kGuarded) {
         float q0, q1;
         split2(q, &q0, &q1);
-        if (kGuarded) {
-            if (use0 && !(q0 >= -170.f && q0 <= 170.f))
-                e0 = dgmr_fm::exp_f_nonpos(-0.5f * q0);
-            if (use1 && !(q1 >= -170.f && q1 <= 170.f))
-                e1 = dgmr_fm::exp_f_nonpos(-0.5f * q1);
-        } else if (fminf(q0, q1) < -170.f) { // rounding of a long thin splat far away; q <= q_cut < 100 where it is used
+        if (use0 && !(q0 >= -170.f && q0 <= 170.f))
             e0 = dgmr_fm::exp_f_nonpos(-0.5f * q0);
+        if (use1 && !(q1 >= -170.f && q1 <= 170.f))
             e1 = dgmr_fm::exp_f_nonpos(-0.5f * q1);
-        }
     }
     const float og0 = op * e0, og1 = op * e1;
     float al0 = min_f(0.99f, og0), al1 = min_f(0.99f, og1);
@@ -588,8 +798,8 @@ __device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, f
 }
 
 template <class Frames>
-__global__ void __launch_bounds__(kBwdWarps * 32, 6) k_splat_bwd_pixels(const int32_t* __restrict__ ranges, const uint32_t* __restrict__ list,
-    const float4* __restrict__ rec, const float* __restrict__ rgb, double* __restrict__ acc, const uint32_t* __restrict__ tile_order,
+__global__ void __launch_bounds__(kBwdWarps * 32, 5) k_splat_bwd_pixels(const int32_t* __restrict__ ranges, const uint32_t* __restrict__ list,
+    const float4* __restrict__ rec, const float* __restrict__ rgb, uint32_t N, double* __restrict__ acc, const uint32_t* __restrict__ tile_order,
     const __grid_constant__ Frames frames)
 {
     __shared__ float4 s_r0[kBwdWarps][32]; // the blend records: (x, y, a, c), (2b, opacity, q_cut, list index as int bits)
@@ -619,10 +829,10 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 6) k_splat_bwd_pixels(const in
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             g[h][c] = inside ? f.grad_fb[c * plane + pix] : 0.f;
-            plain = plain && bwd_plain(g[h][c]);
+            plain = plain && plain_value(g[h][c]);
         }
         bg[h] = T[h] * ((f.bg0 * g[h][0] + f.bg1 * g[h][1]) + f.bg2 * g[h][2]);
-        plain = plain && bwd_plain(bg[h]);
+        plain = plain && plain_value(bg[h]);
     }
     p.Tr = f2(T[0], T[1]);
     p.a0 = p.a1 = p.a2 = f2(0.f);
@@ -648,24 +858,29 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 6) k_splat_bwd_pixels(const in
         if (adds && held_id != 0xffffffffu && total != 0.f)
             atomicAdd(acc + size_t(held_id) * 9 + my_slot, double(total));
     };
+    ListWalk next;
+    next.id = ListWalk::entry(list + b, end - 32 + lane, 0, end);
+    next.later = ListWalk::entry(list + b, end - 64 + lane, 0, end);
+    next.request(rec, rgb, N);
     for (int32_t hi = end; hi > 0; hi -= 32) {
         // the batch's records that can reach a pixel of this quarter (the
         // forward's exact rectangle cull), compacted in list order with their
         // list positions; the others add nothing to any pixel here
-        const int32_t k = (hi > 32 ? hi - 32 : 0) + lane;
+        const int32_t k = hi - 32 + lane;
         bool keep = false, fine = true;
-        float4 r0, r1, c;
-        if (k < hi) {
-            const uint32_t id = list[b + k];
-            r0 = rec[2 * size_t(id)];
-            r1 = rec[2 * size_t(id) + 1];
+        const float4 r0 = next.r0;
+        float4 r1 = next.r1;
+        const uint32_t id = next.id;
+        const float4 c = make_float4(next.c0, next.c1, next.c2, __uint_as_float(id));
+        next.id = next.later;
+        next.later = ListWalk::entry(list + b, k - 64, 0, end);
+        next.request(rec, rgb, N);
+        if (id < N) {
             const float qmin = rect_min_q(r0.x, r0.y, r0.z, 0.5f * r1.x, r0.w, fx0, fx1, fy0, fy1);
             keep = !(qmin > r1.z * 1.001f + 0.01f);
             if (keep) {
                 r1.w = __int_as_float(k);
-                c = make_float4(rgb[3 * size_t(id)], rgb[3 * size_t(id) + 1], rgb[3 * size_t(id) + 2], __uint_as_float(id));
-                fine = bwd_plain(((fabsf(r0.x) + fabsf(r0.y)) + fabsf(r1.x)) + (fabsf(r0.z) + fabsf(r0.w)), kBwdPlainGeometry) && bwd_plain(r1.y)
-                    && bwd_plain((fabsf(c.x) + fabsf(c.y)) + fabsf(c.z));
+                fine = plain_record(r0, r1, c, fx0, fy0);
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
@@ -717,12 +932,12 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 6) k_splat_bwd_pixels(const in
 
 // The per-pixel adjoint over n_tiles tiles.
 template <class Frames>
-void launch_blend_bwd(uint32_t n_tiles, const int32_t* ranges, const uint32_t* list, const float4* rec, const float* rgb, double* acc,
+void launch_blend_bwd(uint32_t n_tiles, const int32_t* ranges, const uint32_t* list, const float4* rec, const float* rgb, uint32_t N, double* acc,
     const uint32_t* tile_order, const Frames& frames, cudaStream_t s)
 {
     if (n_tiles == 0)
         return;
-    k_splat_bwd_pixels<Frames><<<n_tiles, kBwdWarps * 32, 0, s>>>(ranges, list, rec, rgb, acc, tile_order, frames);
+    k_splat_bwd_pixels<Frames><<<n_tiles, kBwdWarps * 32, 0, s>>>(ranges, list, rec, rgb, N, acc, tile_order, frames);
 }
 
 struct SplatBwdGauss {
@@ -1202,7 +1417,7 @@ dgmr_status dgmr_splat_backward(const dgmr_scene* scene, const dgmr_camera* came
     const CameraT<float> cam = make_camera<float>(*camera);
     const int par = tile_sort_parity(super_count(cam.gx, cam.gy));
     cudaMemsetAsync(L.grad_acc, 0, size_t(N) * 9 * sizeof(double), s);
-    launch_blend_bwd(cam.gx * cam.gy, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, L.grad_acc, L.tile_order,
+    launch_blend_bwd(cam.gx * cam.gy, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, N, L.grad_acc, L.tile_order,
         single_frame(cam, nullptr, L, grad_framebuffer), s);
     SplatBwdGauss p { N, static_cast<const float*>(scene->centroids), static_cast<const float*>(scene->sh), scene->sh_stride, scene->sh_degree,
         static_cast<const float*>(scene->weights), static_cast<const float*>(scene->scales), static_cast<const float*>(scene->rotations), L.clamped,
@@ -1428,7 +1643,7 @@ dgmr_status dgmr_splat_batch_backward(const dgmr_scene* scenes, int32_t n_scenes
         return DGMR_OK;
     const int par = tile_sort_parity(plan.tab.n_stiles);
     cudaMemsetAsync(L.grad_acc, 0, size_t(G) * 9 * sizeof(double), s);
-    launch_blend_bwd(plan.tab.n_tiles, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, L.grad_acc, L.tile_order, plan.tab, s);
+    launch_blend_bwd(plan.tab.n_tiles, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, G, L.grad_acc, L.tile_order, plan.tab, s);
     SplatBwdGauss state { 0, nullptr, nullptr, 1, 0, nullptr, nullptr, nullptr, L.clamped, L.tiles_touched, L.grad_acc, nullptr, nullptr, nullptr, nullptr,
         nullptr, Formulation::Ots };
     k_batch_bwd_gaussians<<<(n_scene_gaussians + 127) / 128, 128, 0, s>>>(state, plan.tab);
