@@ -192,6 +192,8 @@ _SIGNATURES = {
     "dgmr_server_now": (C.c_double, [C.c_void_p]),
     "dgmr_server_get_stats": (C.c_int, [C.c_void_p, C.POINTER(ServerStats)]),
     "dgmr_server_destroy": (C.c_int, [C.c_void_p]),
+    "dgmr_camera_read": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.POINTER(Camera),
+                                   C.c_void_p]),
     "dgmr_status_string": (C.c_char_p, [C.c_int]),
     "dgmr_version": (C.c_char_p, []),
     "dgmr_launch_count": (C.c_uint64, []),
@@ -274,11 +276,34 @@ def _host_values(t, n: int) -> list[float]:
     return [float(v) for v in np.asarray(t, dtype=np.float64).reshape(-1)[:n]]
 
 
+def _read_device_camera(c: Camera, tensors) -> bool:
+    """Fills the camera's arrays from four tensors of one dtype on the current
+    device, with one wait on its current stream; False where they are anything
+    else (each array is then read on its own)."""
+    first = tensors[0]
+    if not isinstance(first, torch.Tensor) or not first.is_cuda or first.dtype not in (torch.float32, torch.float64):
+        return False
+    if first.device.index != torch.cuda.current_device():
+        return False
+    for t, n in zip(tensors, (16, 16, 3, 3)):
+        if not isinstance(t, torch.Tensor) or t.device != first.device or t.dtype != first.dtype or t.numel() < n:
+            return False
+    flat = [t.detach().reshape(-1) for t in tensors]
+    flat = [t if t.is_contiguous() else t.contiguous() for t in flat]
+    check(lib().dgmr_camera_read(*[t.data_ptr() for t in flat], dtype_code(first.dtype), C.byref(c), stream_handle()),
+          "camera read")
+    return True
+
+
 def make_camera(view, proj, campos, background, width: int, height: int, tan_fovx: float, tan_fovy: float,
                 cov_scale_multiplier: float = 1.0) -> Camera:
     """view/proj in the torch layout of the reference (row i = glm column i)."""
     c = Camera()
     c.width, c.height = int(width), int(height)
+    c.tan_fovx, c.tan_fovy = float(tan_fovx), float(tan_fovy)
+    c.cov_scale_multiplier = float(cov_scale_multiplier)
+    if _read_device_camera(c, (view, proj, campos, background)):
+        return c
     v = _host_values(view, 16)
     p = _host_values(proj, 16)
     for i in range(16):
@@ -289,6 +314,4 @@ def make_camera(view, proj, campos, background, width: int, height: int, tan_fov
     for i in range(3):
         c.campos[i] = cp[i]
         c.background[i] = bg[i]
-    c.tan_fovx, c.tan_fovy = float(tan_fovx), float(tan_fovy)
-    c.cov_scale_multiplier = float(cov_scale_multiplier)
     return c

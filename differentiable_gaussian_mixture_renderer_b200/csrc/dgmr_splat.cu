@@ -1,6 +1,7 @@
 // Tile-based EWA splat renderer: forward (src/dgmr/splat_forward.cu:30-338)
 // and a reverse-order backward (no reference kernel), behind the C ABI of
 // include/dgmr_b200.h.
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <mutex>
@@ -1739,4 +1740,62 @@ extern "C" dgmr_status dgmr_splat_forward_noalloc(const dgmr_scene* scene, const
         || cudaStreamSynchronize(s) != cudaSuccess)
         return DGMR_ERR_CUDA;
     return (flags & DGMR_FLAG_PAIR_OVERFLOW) ? DGMR_ERR_PAIR_OVERFLOW : DGMR_OK;
+}
+
+// ---------------------------------------------------------------------------
+// A camera on the device, read by the host.
+
+namespace {
+
+constexpr int kCameraValues = 16 + 16 + 3 + 3;
+static_assert(offsetof(dgmr_camera, proj) == offsetof(dgmr_camera, view) + 16 * sizeof(double)
+        && offsetof(dgmr_camera, campos) == offsetof(dgmr_camera, proj) + 16 * sizeof(double)
+        && offsetof(dgmr_camera, background) == offsetof(dgmr_camera, campos) + 3 * sizeof(double),
+    "the four arrays follow one another");
+
+// pinned host memory that the kernel writes: one block per thread, kept until the thread ends
+struct CameraStaging {
+    double* host = nullptr;
+    ~CameraStaging()
+    {
+        if (host)
+            cudaFreeHost(host);
+    }
+};
+
+template <class T>
+__global__ void k_camera_read(const T* __restrict__ view, const T* __restrict__ proj, const T* __restrict__ campos, const T* __restrict__ background,
+    double* __restrict__ out)
+{
+    const int i = threadIdx.x;
+    if (i < kCameraValues)
+        out[i] = double(i < 16 ? view[i] : i < 32 ? proj[i - 16] : i < 35 ? campos[i - 32] : background[i - 35]);
+}
+
+} // namespace
+
+extern "C" dgmr_status dgmr_camera_read(const void* view, const void* proj, const void* campos, const void* background, int32_t dtype, dgmr_camera* camera,
+    dgmr_stream stream)
+{
+    if (!view || !proj || !campos || !background || !camera || (dtype != DGMR_F32 && dtype != DGMR_F64))
+        return DGMR_ERR_BAD_ARG;
+    static thread_local CameraStaging staging;
+    if (!staging.host
+        && cudaHostAlloc(reinterpret_cast<void**>(&staging.host), kCameraValues * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        staging.host = nullptr;
+        cudaGetLastError();
+        return DGMR_ERR_CUDA;
+    }
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    if (dtype == DGMR_F32)
+        k_camera_read<<<1, 64, 0, s>>>(static_cast<const float*>(view), static_cast<const float*>(proj), static_cast<const float*>(campos),
+            static_cast<const float*>(background), staging.host);
+    else
+        k_camera_read<<<1, 64, 0, s>>>(static_cast<const double*>(view), static_cast<const double*>(proj), static_cast<const double*>(campos),
+            static_cast<const double*>(background), staging.host);
+    note_launch();
+    if (launch_status() != DGMR_OK || cudaStreamSynchronize(s) != cudaSuccess)
+        return DGMR_ERR_CUDA;
+    std::memcpy(camera->view, staging.host, kCameraValues * sizeof(double));
+    return DGMR_OK;
 }

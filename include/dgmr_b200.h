@@ -471,6 +471,13 @@ dgmr_status dgmr_server_get_stats(const dgmr_server* server, dgmr_server_stats* 
 /* Waits for work in flight, frees the server's memory. */
 dgmr_status dgmr_server_destroy(dgmr_server* server);
 
+/* Reads a camera that lives on the device: view and proj (16 values each),
+ * campos and background (3 each), contiguous device arrays of `dtype`
+ * (DGMR_F32 / DGMR_F64), into the struct's fields of the same names, and waits for
+ * the stream.  One small kernel instead of four copies, each waited for. */
+dgmr_status dgmr_camera_read(const void* view, const void* proj, const void* campos, const void* background, int32_t dtype, dgmr_camera* camera,
+    dgmr_stream stream);
+
 /* ---------------------------------------------------------------- misc */
 const char* dgmr_status_string(dgmr_status status);
 /* Library version, e.g. "dgmr_b200 0.1 sm_100a". */
