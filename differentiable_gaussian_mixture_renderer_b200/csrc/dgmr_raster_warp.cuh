@@ -10,10 +10,13 @@
 //    j+1 and a warp minimum picks the cheapest (the first of equals).
 //    The transmittance in front of each slot is the same left-to-right
 //    product as the one-thread sizer's, so every merge decision matches it.
-//  * Pass B: for each Gaussian of the tile, lane q evaluates the CDF at its
-//    bin's right border (the left one is its neighbour's) and accumulates its
-//    bin's four masses and border values in registers -- per bin the same
-//    Gaussian order and operations as the one-thread loop.
+//  * Pass B: the tile's Gaussians that reach the bins are packed into shared
+//    memory, what depends on the Gaussian alone (its CDF at 0, its value at the
+//    far end) computed by the lane that loaded it; then, two Gaussians at a time
+//    as the halves of packed floats, lane q evaluates the CDF at its bin's right
+//    border (the left one is its neighbour's) and accumulates its bin's four
+//    masses and border values in registers -- per bin the same Gaussian order and
+//    operations as the one-thread loop.
 //  * Blend: lane q fits its bin and integrates its 256 steps from T = 1; the
 //    bins' colours and transmittances are then chained in bin order.
 // The one-thread-per-pixel kernel this replaces kept ~1 KB of bins and the
@@ -22,13 +25,36 @@
 // leave at once.
 #pragma once
 
+#include "dgmr_f32x2.cuh"
+
 namespace dgmr {
 
 constexpr unsigned kVrRayWarps = 4; // rays per block
 
-// eval_exponential_1d as a call: the warp kernel is large enough to stall on
-// instruction fetch with every exp inlined (same arithmetic, same bits)
-__device__ __noinline__ float eval_exponential_1d_call(float c, float var, float x) { return eval_exponential_1d(c, var, x); }
+// eval_exponential_1d of two Gaussians at one position; nc = -centre
+__device__ __forceinline__ F2 eval2_exponential_1d(F2 nc, float var0, float var1, float x)
+{
+    const F2 dx = add2(f2(x), nc);
+    float a0, a1;
+    split2(mul2(f2(-0.5f), mul2(dx, dx)), &a0, &a1);
+    const float x0 = a0 / var0, x1 = a1 / var1;
+    float e0, e1;
+    split2(exp2_nonpos(f2(x0, x1)), &e0, &e1);
+    // past the packed exp's range: zero, or (NaN, the subnormal results) the scalar one
+    if (!(x0 >= -87.f && x0 <= 0.f))
+        e0 = x0 < -104.f ? 0.f : dgmr_fm::exp_f(x0);
+    if (!(x1 >= -87.f && x1 <= 0.f))
+        e1 = x1 < -104.f ? 0.f : dgmr_fm::exp_f(x1);
+    return f2(e0, e1);
+}
+
+// A Gaussian of pass B as every lane reads it.
+struct alignas(16) VrStaged {
+    float centre, inv_sd, var, weight;
+    float cdf0, last; // CDF at 0; weight times the value at the far end
+    float r, g;
+    float b, one, pad0, pad1;
+};
 
 struct RayEntryVr {
     uint32_t id;
@@ -37,10 +63,12 @@ struct RayEntryVr {
     float mass;
 };
 
-// the sizer's slot held by this lane, and the ray-wide totals
+// the sizer's slot held by this lane, and the ray-wide totals; front: the
+// transmittance in front of the slot, up to date for slots 0 to front_ok
 struct WarpBinSizer {
-    float mass, border, sd;
+    float mass, border, sd, front;
     float total, far, full_mass, sigma;
+    unsigned front_ok;
 };
 
 __device__ __forceinline__ void wbs_init(WarpBinSizer& s, float sigma, float transmission_threshold)
@@ -48,6 +76,8 @@ __device__ __forceinline__ void wbs_init(WarpBinSizer& s, float sigma, float tra
     s.mass = 0.f;
     s.border = 1.f / 0.f;
     s.sd = 0.f;
+    s.front = 1.f;
+    s.front_ok = 0u;
     s.total = 0.f;
     s.far = 0.f;
     s.sigma = sigma;
@@ -84,17 +114,21 @@ __device__ __forceinline__ void wbs_add(WarpBinSizer& s, unsigned lane, float ma
         s.border = centre;
         s.sd = sd;
     }
+    s.front_ok = min(s.front_ok, p);
     if (!(__shfl_sync(kFull, s.mass, kVrBins - 1) > 0.f))
         return;
-    // transmittance in front of each slot: the one-thread sizer's left-to-right product
+    // transmittance in front of each slot: the one-thread sizer's left-to-right
+    // product, continued from the last slot that it holds for
     const float ex = dgmr_fm::exp_f(-s.mass);
-    float run = 1.f, front = 1.f;
+    float run = __shfl_sync(kFull, s.front, int(s.front_ok));
 #pragma unroll 1
-    for (unsigned i = 0; i + 1 < kVrBins; ++i) {
+    for (unsigned i = s.front_ok; i + 1 < kVrBins; ++i) {
         run = run * __shfl_sync(kFull, ex, int(i));
         if (lane == i + 1)
-            front = run;
+            s.front = run;
     }
+    s.front_ok = kVrBins - 1;
+    const float front = s.front;
     // lane j < 31: the merge of slots j and j + 1 and its cost
     const float nm = __shfl_down_sync(kFull, s.mass, 1), nb = __shfl_down_sync(kFull, s.border, 1), nsd = __shfl_down_sync(kFull, s.sd, 1);
     const float nfront = __shfl_down_sync(kFull, front, 1);
@@ -115,6 +149,7 @@ __device__ __forceinline__ void wbs_add(WarpBinSizer& s, unsigned lane, float ma
     if (!(lo < 1.f / 0.f))
         return;
     const unsigned pick = unsigned(__ffs(int(__ballot_sync(kFull, key == lo))) - 1);
+    s.front_ok = pick;
     // the merged lobe takes slot pick, the slots behind it move one left, the last stays
     if (lane == pick) {
         s.mass = m_mass;
@@ -165,10 +200,16 @@ __device__ __forceinline__ RayEntryVr load_vr_entry(const VrRender& a, int32_t k
     return en;
 }
 
-// vol_raster_forward.cu:253-517, one warp per ray
-__global__ void __launch_bounds__(kVrRayWarps * 32) k_vr_render_warp(VrRender a, CameraT<float> cam)
+// vol_raster_forward.cu:253-517, one warp per ray.  Bound by instruction issue
+// (30,000 warp instructions per ray at 100k, 512^2, a third of them the 256
+// integration steps).  Against a Gaussian at a time in pass B (its CDF at 0 and
+// its far value evaluated by one lane while 31 waited), a scalar integration and
+// the whole product of transmittances per added Gaussian: 10.40 -> 8.48 ms, mean
+// of four cameras; 56 registers and nine blocks per SM instead of 70: 8.29.
+__global__ void __launch_bounds__(kVrRayWarps * 32, 9) k_vr_render_warp(VrRender a, CameraT<float> cam)
 {
     constexpr unsigned kFull = 0xffffffffu;
+    __shared__ VrStaged staged[kVrRayWarps][32];
     const unsigned lane = threadIdx.x & 31u;
     const unsigned per_tile = kTilePixels / kVrRayWarps;
     const unsigned tile = blockIdx.x / per_tile;
@@ -201,7 +242,11 @@ __global__ void __launch_bounds__(kVrRayWarps * 32) k_vr_render_warp(VrRender a,
                 centre = g.centre;
                 sd = dgmr_fm::sqrt_f(g.C + 0.f);
                 reach = centre + sd * kVrRelevanceSigma;
-                on_ray = mor * (RasterBinSizer<kVrBins>::cdf(centre, sd, reach) - RasterBinSizer<kVrBins>::cdf(centre, sd, 0.f));
+                // RasterBinSizer::cdf at both ends
+                const float scale = sd * 1.41421356237309505f;
+                float at_reach, at_zero;
+                split2(mul2(f2(0.5f), add2(f2(1.f), erf2(f2((reach - centre) / scale, (0.f - centre) / scale)))), &at_reach, &at_zero);
+                on_ray = mor * (at_reach - at_zero);
             }
         }
         uint32_t m = __ballot_sync(kFull, ok);
@@ -224,56 +269,85 @@ __global__ void __launch_bounds__(kVrRayWarps * 32) k_vr_render_warp(VrRender a,
     float res0 = 0.f, res1 = 0.f, res2 = 0.f, transparency = 1.f; // the final colour adds T = 1 x background in Full and Bins mode
     if (a.mode == DGMR_RENDER_FULL) {
         // pass B: bin masses and border values of every Gaussian of the tile
-        float bm[4] = { 0.f, 0.f, 0.f, 0.f }, be[4] = { 0.f, 0.f, 0.f, 0.f }, be_last[4] = { 0.f, 0.f, 0.f, 0.f };
+        VrStaged* row = staged[threadIdx.x >> 5];
+        F2 bm_rg = f2(0.f), bm_bm = f2(0.f), be_rg = f2(0.f), be_bm = f2(0.f), last_rg = f2(0.f), last_bm = f2(0.f); // (r, g), (b, mass)
         const float max_distance = sz.far;
+        const F2 ends = f2(end);
         for (int32_t base = b; base < e; base += 32) {
-            float centre = 0.f, inv_sd = 0.f, variance = 0.f, weight = 0.f;
-            V3<float> rgb = { 0.f, 0.f, 0.f };
+            VrStaged st;
             bool ok = false;
             if (base + int32_t(lane) < e) {
                 const RayEntryVr en = load_vr_entry(a, base + int32_t(lane));
                 const Gauss1d<float> g = intersect_with_ray_inv_C(en.mu, en.Q, o, d);
-                centre = g.centre;
-                variance = g.C + 0.f;
-                const float sd = dgmr_fm::sqrt_f(variance);
-                inv_sd = 1.f / sd;
-                weight = g.weight * en.mass;
-                ok = !(variance <= 0.f || dgmr_fm::isnan_f(variance) || dgmr_fm::isnan_f(weight) || weight > 100000.f)
-                    && !(weight * (cdf_inv_SD_inline(centre, inv_sd, max_distance) - cdf_inv_SD_inline(centre, inv_sd, 0.f)) <= 0.001f);
-                if (ok)
-                    rgb = { a.rgb[3 * size_t(en.id)], a.rgb[3 * size_t(en.id) + 1], a.rgb[3 * size_t(en.id) + 2] };
+                st.centre = g.centre;
+                st.var = g.C + 0.f;
+                const float sd = dgmr_fm::sqrt_f(st.var);
+                st.inv_sd = 1.f / sd;
+                st.weight = g.weight * en.mass;
+                ok = !(st.var <= 0.f || dgmr_fm::isnan_f(st.var) || dgmr_fm::isnan_f(st.weight) || st.weight > 100000.f);
+                if (ok) {
+                    float far;
+                    split2(cdf2_inv_SD(f2(-st.centre), f2(st.inv_sd), f2(max_distance, 0.f)), &far, &st.cdf0);
+                    ok = !(st.weight * (far - st.cdf0) <= 0.001f);
+                }
+                if (ok) {
+                    st.last = st.weight * eval_exponential_1d(st.centre, st.var, max_distance);
+                    st.r = a.rgb[3 * size_t(en.id)];
+                    st.g = a.rgb[3 * size_t(en.id) + 1];
+                    st.b = a.rgb[3 * size_t(en.id) + 2];
+                    st.one = 1.f;
+                }
             }
-            uint32_t m = __ballot_sync(kFull, ok);
-            while (m) {
-                const int j = __ffs(int(m)) - 1;
-                m &= m - 1u;
-                const float cj = __shfl_sync(kFull, centre, j), ij = __shfl_sync(kFull, inv_sd, j);
-                const float vj = __shfl_sync(kFull, variance, j), wj = __shfl_sync(kFull, weight, j);
-                const float r = __shfl_sync(kFull, rgb.x, j), gg = __shfl_sync(kFull, rgb.y, j), bb = __shfl_sync(kFull, rgb.z, j);
-                const float cdf_end = cdf_inv_SD(cj, ij, end);
-                const float cdf_left = __shfl_up_sync(kFull, cdf_end, 1);
-                const float cdf_start = lane == 0 ? cdf_inv_SD(cj, ij, 0.f) : cdf_left;
-                const float mass = (cdf_end - cdf_start) * wj;
-                if (!(mass < 0.0001f)) {
-                    bm[0] = bm[0] + r * mass;
-                    bm[1] = bm[1] + gg * mass;
-                    bm[2] = bm[2] + bb * mass;
-                    bm[3] = bm[3] + mass;
-                    const float ev = wj * eval_exponential_1d_call(cj, vj, begin);
-                    be[0] = be[0] + r * ev;
-                    be[1] = be[1] + gg * ev;
-                    be[2] = be[2] + bb * ev;
-                    be[3] = be[3] + ev;
+            const uint32_t m = __ballot_sync(kFull, ok);
+            if (!m)
+                continue;
+            const int n = __popc(m);
+            __syncwarp(); // the last batch is read
+            if (ok)
+                row[__popc(m & ((1u << lane) - 1u))] = st;
+            if ((n & 1) && lane == 0) // an odd one's partner: no weight, no mass
+                row[n] = VrStaged { 0.f, 1.f, 1.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f };
+            __syncwarp();
+            for (int j = 0; j < n; j += 2) {
+                const VrStaged &g0 = row[j], &g1 = row[j + 1];
+                const F2 nc = f2(-g0.centre, -g1.centre);
+                const F2 cdf_end = cdf2_inv_SD(nc, f2(g0.inv_sd, g1.inv_sd), ends);
+                float end0, end1;
+                split2(cdf_end, &end0, &end1);
+                const float left0 = __shfl_up_sync(kFull, end0, 1), left1 = __shfl_up_sync(kFull, end1, 1);
+                const float mass0 = (end0 - (lane == 0 ? g0.cdf0 : left0)) * g0.weight, mass1 = (end1 - (lane == 0 ? g1.cdf0 : left1)) * g1.weight;
+                const bool has0 = !(mass0 < 0.0001f), has1 = !(mass1 < 0.0001f);
+                const F2 rg0 = f2(g0.r, g0.g), rg1 = f2(g1.r, g1.g), bm0 = f2(g0.b, g0.one), bm1 = f2(g1.b, g1.one);
+                if (has0 || has1) {
+                    float ev0, ev1;
+                    split2(mul2(f2(g0.weight, g1.weight), eval2_exponential_1d(nc, g0.var, g1.var, begin)), &ev0, &ev1);
+                    if (has0) {
+                        bm_rg = add2(bm_rg, mul2_rounded(rg0, f2(mass0)));
+                        bm_bm = add2(bm_bm, mul2_rounded(bm0, f2(mass0)));
+                        be_rg = add2(be_rg, mul2_rounded(rg0, f2(ev0)));
+                        be_bm = add2(be_bm, mul2_rounded(bm0, f2(ev0)));
+                    }
+                    if (has1) {
+                        bm_rg = add2(bm_rg, mul2_rounded(rg1, f2(mass1)));
+                        bm_bm = add2(bm_bm, mul2_rounded(bm1, f2(mass1)));
+                        be_rg = add2(be_rg, mul2_rounded(rg1, f2(ev1)));
+                        be_bm = add2(be_bm, mul2_rounded(bm1, f2(ev1)));
+                    }
                 }
-                if (lane == kVrBins - 1) {
-                    const float ev = wj * eval_exponential_1d_call(cj, vj, max_distance);
-                    be_last[0] = be_last[0] + r * ev;
-                    be_last[1] = be_last[1] + gg * ev;
-                    be_last[2] = be_last[2] + bb * ev;
-                    be_last[3] = be_last[3] + ev;
-                }
+                // the values at the far end (read by the last bin's lane)
+                last_rg = add2(last_rg, mul2_rounded(rg0, f2(g0.last)));
+                last_bm = add2(last_bm, mul2_rounded(bm0, f2(g0.last)));
+                last_rg = add2(last_rg, mul2_rounded(rg1, f2(g1.last)));
+                last_bm = add2(last_bm, mul2_rounded(bm1, f2(g1.last)));
             }
         }
+        float bm[4], be[4], be_last[4];
+        split2(bm_rg, &bm[0], &bm[1]);
+        split2(bm_bm, &bm[2], &bm[3]);
+        split2(be_rg, &be[0], &be[1]);
+        split2(be_bm, &be[2], &be[3]);
+        split2(last_rg, &be_last[0], &be_last[1]);
+        split2(last_bm, &be_last[2], &be_last[3]);
         // blend: lane q fits bin q (the split of a bin's mass between its halves is
         // 0.5 for every bin and channel, vol_raster_forward.cu:473) and integrates
         // it from T = 1; then the bins are chained in order
@@ -290,14 +364,27 @@ __global__ void __launch_bounds__(kVrRayWarps * 32) k_vr_render_warp(VrRender a,
             const FunctionGroup<float> f = create_approximation(half, bm, be, right, t_right);
             const float dt = f.t_right / float(kVrStepsPerBin);
             float t = dt / 2.f;
+            // FunctionGroup::sample of channels (r, g) and (b, mass) as packed halves
+            const F2 d01 = f2(f.d0[0], f.d0[1]), d23 = f2(f.d0[2], f.d0[3]), k01 = f2(f.k0[0], f.k0[1]), k23 = f2(f.k0[2], f.k0[3]);
+            const F2 b01 = add2(d01, mul2_rounded(f2(f.t1[0], f.t1[1]), k01)), b23 = add2(d23, mul2_rounded(f2(f.t1[2], f.t1[3]), k23));
+            const F2 n01 = f2(-f.t2[0], -f.t2[1]), n23 = f2(-f.t2[2], -f.t2[3]), r01 = f2(f.k2[0], f.k2[1]), r23 = f2(f.k2[2], f.k2[3]);
+            F2 l01 = f2(0.f);
             for (unsigned s = 0; s < kVrStepsPerBin; ++s) {
-                const float e0 = f.sample(0, t), e1 = f.sample(1, t), e2 = f.sample(2, t), e3 = f.sample(3, t);
-                l0 = l0 + (e0 * cur) * dt;
-                l1 = l1 + (e1 * cur) * dt;
-                l2 = l2 + (e2 * cur) * dt;
-                cur = cur * max_f(0.f, 1.f - e3 * dt);
+                const F2 tt = f2(t);
+                float lo[4], hi[4], ev[4];
+                split2(add2(d01, mul2_rounded(k01, tt)), &lo[0], &lo[1]);
+                split2(add2(d23, mul2_rounded(k23, tt)), &lo[2], &lo[3]);
+                split2(add2(b01, mul2_rounded(add2(tt, n01), r01)), &hi[0], &hi[1]);
+                split2(add2(b23, mul2_rounded(add2(tt, n23), r23)), &hi[2], &hi[3]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    ev[c] = t <= f.t1[c] ? lo[c] : t <= f.t2[c] ? 0.f : hi[c];
+                l01 = add2(l01, mul2_rounded(mul2(f2(ev[0], ev[1]), f2(cur)), f2(dt)));
+                l2 = l2 + (ev[2] * cur) * dt;
+                cur = cur * max_f(0.f, 1.f - ev[3] * dt);
                 t = t + dt;
             }
+            split2(l01, &l0, &l1);
         }
         float tr = 1.f;
 #pragma unroll 1
