@@ -252,13 +252,6 @@ static __global__ void k_super_counts(const uint32_t* __restrict__ perm, const u
     rect_hi[j] = r.x1 | (r.y1 << 16);
 }
 
-// n_sort[1] = super-tile entries to sort = min(total, cap)
-static __global__ void k_super_total(const uint32_t* __restrict__ off_sorted, uint32_t N, uint32_t cap, uint32_t* __restrict__ n_sort)
-{
-    const uint32_t n = N ? off_sorted[N - 1] : 0u;
-    n_sort[1] = n < cap ? n : cap;
-}
-
 // Super-tile entries in depth order: for the j-th Gaussian by depth, one entry
 // per super-tile its rectangle touches, row-major: key = super-tile id << 12 |
 // the rectangle's part inside it, value = the Gaussian.  The 32
@@ -399,6 +392,48 @@ static __global__ void __launch_bounds__(1024) k_chunk_plan(const int32_t* __res
     if (threadIdx.x == 0) {
         chunk_base[n_super] = carry;
         n_sort[2] = carry;
+    }
+}
+
+// The same, and the super-tiles' ranges, from the digit totals of a sort whose one
+// pass covered all their bits (digit = super-tile, at most 256): without the
+// pass over the sorted keys that finds the ranges (k_tile_ranges, 5.7 us for 1.7M
+// entries).  One block of kSortBins threads.
+static __global__ void __launch_bounds__(kSortBins) k_super_plan(const uint32_t* __restrict__ digit_total, uint32_t n_super, int32_t* __restrict__ super_ranges,
+    uint32_t* __restrict__ chunk_base, uint32_t* __restrict__ n_sort)
+{
+    __shared__ uint32_t len_tot[kSortWarps], chunk_tot[kSortWarps];
+    const uint32_t s = threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t len = s < n_super ? digit_total[s] : 0u, chunks = (len + kChunk - 1) / kChunk;
+    uint32_t x = len, y = chunks;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t xs = __shfl_up_sync(0xffffffffu, x, o), ys = __shfl_up_sync(0xffffffffu, y, o);
+        if (lane >= o) {
+            x += xs;
+            y += ys;
+        }
+    }
+    if (lane == 31) {
+        len_tot[warp] = x;
+        chunk_tot[warp] = y;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w)
+        if (w < warp) {
+            x += len_tot[w];
+            y += chunk_tot[w];
+        }
+    if (s < n_super) {
+        super_ranges[2 * s] = len ? int32_t(x - len) : 0;
+        super_ranges[2 * s + 1] = len ? int32_t(x) : 0;
+        chunk_base[s] = y - chunks;
+        if (s == n_super - 1) {
+            chunk_base[n_super] = y;
+            n_sort[2] = y;
+        }
     }
 }
 
@@ -570,7 +605,7 @@ static __global__ void __launch_bounds__(kSuperTiles* kPrefixParts) k_chunk_pref
 }
 
 // splat_forward.cu:218-239: [start, end) of each tile's run, (0, 0) for an
-// empty tile; clamped to the pair capacity.
+// empty tile; clamped to the pair capacity (k_scan_single writes them itself).
 static __global__ void k_tile_ranges_from_counts(const uint32_t* __restrict__ tile_total, const uint32_t* __restrict__ tile_incl, uint32_t n_tiles,
     uint32_t cap, int32_t* __restrict__ ranges)
 {
@@ -812,32 +847,37 @@ inline int run_binning_grids(uint32_t N, uint32_t n_tiles, uint32_t n_super, con
     uint32_t* rect_hi = dpar ? b.perm : b.perm_tmp;
     const uint32_t blocks = (N + 255) / 256;
     k_super_counts<T, Grids><<<blocks, 256, 0, s>>>(perm, tiles_touched, rects, xy, N, b.cnt_sorted, rect_lo, rect_hi, stats, grids);
-    inclusive_scan_u32(b.cnt_sorted, b.off_sorted, N, b.scan_tmp, s);
-    k_super_total<<<1, 1, 0, s>>>(b.off_sorted, N, cap, b.n_sort);
-    note_launch(2);
-    cudaMemsetAsync(b.super_ranges, 0, size_t(n_super) * 2 * sizeof(int32_t), s);
-    cudaMemsetAsync(b.tile_total, 0, size_t(n_tiles) * sizeof(uint32_t), s);
+    note_launch();
+    // n_sort[1] = super-tile entries to sort = min(total, cap)
+    inclusive_scan_u32(b.cnt_sorted, b.off_sorted, N, b.scan_tmp, s, ScanTotal { b.n_sort + 1, cap });
     if (cap > 0) {
         k_emit_super<Grids><<<blocks, 256, 0, s>>>(perm, b.cnt_sorted, b.off_sorted, rect_lo, rect_hi, N, cap, b.pair_tile[0], b.pair_val[0], stats, grids);
         note_launch();
         const int spar = radix_sort_pairs(b.pair_tile[0], b.pair_val[0], b.pair_tile[1], b.pair_val[1], b.n_sort + 1, 0, cap,
             kRectBits + int(higher_msb(n_super)), b.sort_tmp, n_sms, s, stats, kRectBits);
-        const uint32_t want = (cap + 255) / 256, limit = uint32_t(n_sms) * 16;
-        k_tile_ranges<<<want < limit ? want : limit, 256, 0, s>>>(b.pair_tile[spar], b.n_sort + 1, b.super_ranges, n_super, stats, kRectBits);
-        k_chunk_plan<<<1, 1024, 0, s>>>(b.super_ranges, n_super, b.chunk_base, b.n_sort);
+        if (int(higher_msb(n_super)) <= 8) {
+            k_super_plan<<<1, kSortBins, 0, s>>>(radix_digit_totals(b.sort_tmp, cap), n_super, b.super_ranges, b.chunk_base, b.n_sort);
+        } else {
+            const uint32_t want = (cap + 255) / 256, limit = uint32_t(n_sms) * 16;
+            cudaMemsetAsync(b.super_ranges, 0, size_t(n_super) * 2 * sizeof(int32_t), s);
+            k_tile_ranges<<<want < limit ? want : limit, 256, 0, s>>>(b.pair_tile[spar], b.n_sort + 1, b.super_ranges, n_super, stats, kRectBits);
+            k_chunk_plan<<<1, 1024, 0, s>>>(b.super_ranges, n_super, b.chunk_base, b.n_sort);
+            note_launch();
+        }
         const ChunkRows rows = chunk_rows(b);
         const uint32_t cgrid = rows.max_chunks < uint32_t(n_sms) * 8 ? rows.max_chunks : uint32_t(n_sms) * 8;
         k_chunk_counts<Grids><<<cgrid, kChunkThreads, 0, s>>>(b.pair_tile[spar], b.pair_val[spar], N, b.super_ranges, b.chunk_base, n_super, b.n_sort, rows,
             stats, grids);
         k_chunk_prefix<Grids><<<n_super, kSuperTiles * kPrefixParts, 0, s>>>(b.chunk_base, n_super, rows, b.tile_total, n_tiles, stats, grids);
-        note_launch(4);
+        note_launch(3);
         if (n_tiles <= kScanSingleMax) {
-            k_scan_single<<<1, 1024, 0, s>>>(b.tile_total, n_tiles, b.tile_incl);
+            k_scan_single<<<1, 1024, 0, s>>>(b.tile_total, n_tiles, b.tile_incl, ScanTotal { nullptr, 0u }, ranges, cap);
             note_launch();
         } else {
             inclusive_scan_u32(b.tile_total, b.tile_incl, n_tiles, b.scan_tmp, s);
+            k_tile_ranges_from_counts<<<(n_tiles + 255) / 256, 256, 0, s>>>(b.tile_total, b.tile_incl, n_tiles, cap, ranges);
+            note_launch();
         }
-        k_tile_ranges_from_counts<<<(n_tiles + 255) / 256, 256, 0, s>>>(b.tile_total, b.tile_incl, n_tiles, cap, ranges);
         static bool smem_set = false; // one opt-in per instantiation, above the 48 KB default
         if (!smem_set) {
             cudaFuncSetAttribute(k_chunk_emit<Grids>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(chunk_emit_smem()));
@@ -845,7 +885,7 @@ inline int run_binning_grids(uint32_t N, uint32_t n_tiles, uint32_t n_super, con
         }
         k_chunk_emit<Grids><<<cgrid, kChunkThreads, chunk_emit_smem(), s>>>(b.pair_tile[spar], b.pair_val[spar], N, b.super_ranges, b.chunk_base, n_super,
             b.n_sort, rows, b.tile_total, b.tile_incl, cap, b.pair_tile[1 - spar], b.pair_val[1 - spar], stats, grids);
-        note_launch(2);
+        note_launch();
     } else {
         cudaMemsetAsync(ranges, 0, size_t(n_tiles) * 2 * sizeof(int32_t), s);
     }
