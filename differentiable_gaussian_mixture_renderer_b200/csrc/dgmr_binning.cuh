@@ -161,6 +161,7 @@ inline int tile_sort_parity(uint32_t n_super)
 
 static __global__ void k_pair_count(const uint32_t* __restrict__ point_offsets, uint32_t N, uint32_t cap, uint32_t* __restrict__ stats, uint32_t* __restrict__ n_sort)
 {
+    chain_start();
     n_sort[4] = 0xffffffffu; // depth-key range, filled by k_key_range
     n_sort[5] = 0u;
     n_sort[6] = 0u; // counter of the blend's tile-order kernel (k_blend_tile_order)
@@ -234,6 +235,7 @@ static __global__ void k_super_counts(const uint32_t* __restrict__ perm, const u
     const T* __restrict__ xy, uint32_t N, uint32_t* __restrict__ cnt_sorted, uint32_t* __restrict__ rect_lo, uint32_t* __restrict__ rect_hi,
     uint32_t* __restrict__ stats, const __grid_constant__ Grids grids)
 {
+    chain_start();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= N)
         return;
@@ -265,6 +267,7 @@ static __global__ void __launch_bounds__(256) k_emit_super(const uint32_t* __res
     const uint32_t* __restrict__ off_sorted, const uint32_t* __restrict__ rect_lo, const uint32_t* __restrict__ rect_hi, uint32_t N, uint32_t cap,
     uint32_t* __restrict__ skey, uint32_t* __restrict__ sval, uint32_t* __restrict__ stats, const __grid_constant__ Grids grids)
 {
+    chain_start();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     if (__all_sync(0xffffffffu, j >= N))
@@ -353,6 +356,7 @@ static __global__ void __launch_bounds__(256) k_emit_super(const uint32_t* __res
 static __global__ void __launch_bounds__(1024) k_chunk_plan(const int32_t* __restrict__ super_ranges, uint32_t n_super, uint32_t* __restrict__ chunk_base,
     uint32_t* __restrict__ n_sort)
 {
+    chain_start();
     __shared__ uint32_t warp_tot[32];
     __shared__ uint32_t carry;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -402,6 +406,7 @@ static __global__ void __launch_bounds__(1024) k_chunk_plan(const int32_t* __res
 static __global__ void __launch_bounds__(kSortBins) k_super_plan(const uint32_t* __restrict__ digit_total, uint32_t n_super, int32_t* __restrict__ super_ranges,
     uint32_t* __restrict__ chunk_base, uint32_t* __restrict__ n_sort)
 {
+    chain_start();
     __shared__ uint32_t len_tot[kSortWarps], chunk_tot[kSortWarps];
     const uint32_t s = threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -517,6 +522,7 @@ static __global__ void __launch_bounds__(kChunkThreads) k_chunk_counts(const uin
     const int32_t* __restrict__ super_ranges, const uint32_t* __restrict__ chunk_base, uint32_t n_super, const uint32_t* __restrict__ n_sort,
     const ChunkRows rows, uint32_t* __restrict__ stats, const __grid_constant__ Grids grids)
 {
+    chain_start();
     __shared__ uint32_t cnt[kSuperTiles];
     uint32_t n_chunks = n_sort[2];
     if (n_chunks > rows.max_chunks) {
@@ -558,6 +564,7 @@ template <class Grids>
 static __global__ void __launch_bounds__(kSuperTiles* kPrefixParts) k_chunk_prefix(const uint32_t* __restrict__ chunk_base, uint32_t n_super,
     const ChunkRows rows, uint32_t* __restrict__ tile_total, uint32_t n_tiles, uint32_t* __restrict__ stats, const __grid_constant__ Grids grids)
 {
+    chain_start();
     __shared__ uint32_t part[kPrefixParts][kSuperTiles];
     const uint32_t s = blockIdx.x;
     const uint32_t k = threadIdx.x % kSuperTiles, q = threadIdx.x / kSuperTiles;
@@ -609,6 +616,7 @@ static __global__ void __launch_bounds__(kSuperTiles* kPrefixParts) k_chunk_pref
 static __global__ void k_tile_ranges_from_counts(const uint32_t* __restrict__ tile_total, const uint32_t* __restrict__ tile_incl, uint32_t n_tiles,
     uint32_t cap, int32_t* __restrict__ ranges)
 {
+    chain_start();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n_tiles)
         return;
@@ -636,6 +644,7 @@ static __global__ void __launch_bounds__(kChunkThreads) k_chunk_emit(const uint3
     const ChunkRows rows, const uint32_t* __restrict__ tile_total, const uint32_t* __restrict__ tile_incl, uint32_t cap, uint32_t* __restrict__ out_tile,
     uint32_t* __restrict__ out_val, uint32_t* __restrict__ stats, const __grid_constant__ Grids grids)
 {
+    chain_start();
     constexpr int kWarps = kChunkThreads / 32;
     extern __shared__ uint32_t stage_val[]; // [kEmitStage]
     uint8_t* stage_k = reinterpret_cast<uint8_t*>(stage_val + kEmitStage); // [kEmitStage]
@@ -748,6 +757,7 @@ inline size_t chunk_emit_smem() { return size_t(kEmitStage) * (sizeof(uint32_t) 
 static __global__ void k_tile_ranges(const uint32_t* __restrict__ tiles_sorted, const uint32_t* __restrict__ n_dev, int32_t* __restrict__ ranges, uint32_t n_tiles,
     uint32_t* __restrict__ stats, int shift)
 {
+    chain_start();
     const uint32_t n = *n_dev;
     // four items per thread and step, every load issued before the first is used
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -789,6 +799,7 @@ static __global__ void k_tile_ranges(const uint32_t* __restrict__ tiles_sorted, 
 // (k_blend_tile_order): there the longest lists saturate early.
 static __global__ void __launch_bounds__(1024) k_tile_order(const int32_t* __restrict__ ranges, uint32_t n_tiles, uint32_t* __restrict__ order)
 {
+    chain_start();
     __shared__ uint32_t count[33];
     __shared__ uint32_t cursor[33];
     if (threadIdx.x < 33)
@@ -820,8 +831,9 @@ static __global__ void __launch_bounds__(1024) k_tile_order(const int32_t* __res
 // preprocess.  n_super = super-tiles of all frames (super_count per frame).
 template <class T, class Grids>
 inline int run_binning_grids(uint32_t N, uint32_t n_tiles, uint32_t n_super, const Grids& grids, const uint32_t* tiles_touched, uint32_t* point_offsets,
-    const int32_t* rects, const T* xy, uint32_t cap, BinningBuffers& b, int32_t* ranges, uint32_t* stats, int n_sms, cudaStream_t s, bool offsets_ready)
+    const int32_t* rects, const T* xy, uint32_t cap, BinningBuffers& b, int32_t* ranges, uint32_t* stats, int n_sms, cudaStream_t stream, bool offsets_ready)
 {
+    const ChainStream s(stream, N <= kChainMost);
     const int par = tile_sort_parity(n_super);
     if (N == 0) {
         cudaMemsetAsync(ranges, 0, size_t(n_tiles) * 2 * sizeof(int32_t), s);
@@ -830,13 +842,13 @@ inline int run_binning_grids(uint32_t N, uint32_t n_tiles, uint32_t n_super, con
     }
     if (!offsets_ready)
         inclusive_scan_u32(tiles_touched, point_offsets, N, b.scan_tmp, s);
-    k_pair_count<<<1, 1, 0, s>>>(point_offsets, N, cap, stats, b.n_sort);
+    launch_chained(k_pair_count, 1, 1, 0, s, point_offsets, N, cap, stats, b.n_sort);
     note_launch();
     // the depth keys of the Gaussians that touch a tile usually span < 2^24
     // values: rebased, the top pass only copies
     {
         const uint32_t want = (N + 255) / 256, limit = uint32_t(n_sms) * 8;
-        k_key_range<<<want < limit ? want : limit, 256, 0, s>>>(b.depth_key, tiles_touched, N, b.n_sort + 4);
+        launch_chained(k_key_range, want < limit ? want : limit, 256, 0, s, b.depth_key, tiles_touched, N, b.n_sort + 4);
         note_launch();
     }
     const int dpar = radix_sort_pairs(b.depth_key, b.perm, b.key_tmp, b.perm_tmp, nullptr, N, N, 32, b.sort_tmp, n_sms, s, stats, 0, b.n_sort + 4,
@@ -846,36 +858,36 @@ inline int run_binning_grids(uint32_t N, uint32_t n_tiles, uint32_t n_super, con
     uint32_t* rect_lo = dpar ? b.depth_key : b.key_tmp;
     uint32_t* rect_hi = dpar ? b.perm : b.perm_tmp;
     const uint32_t blocks = (N + 255) / 256;
-    k_super_counts<T, Grids><<<blocks, 256, 0, s>>>(perm, tiles_touched, rects, xy, N, b.cnt_sorted, rect_lo, rect_hi, stats, grids);
+    launch_chained(k_super_counts<T, Grids>, blocks, 256, 0, s, perm, tiles_touched, rects, xy, N, b.cnt_sorted, rect_lo, rect_hi, stats, grids);
     note_launch();
     // n_sort[1] = super-tile entries to sort = min(total, cap)
     inclusive_scan_u32(b.cnt_sorted, b.off_sorted, N, b.scan_tmp, s, ScanTotal { b.n_sort + 1, cap });
     if (cap > 0) {
-        k_emit_super<Grids><<<blocks, 256, 0, s>>>(perm, b.cnt_sorted, b.off_sorted, rect_lo, rect_hi, N, cap, b.pair_tile[0], b.pair_val[0], stats, grids);
+        launch_chained(k_emit_super<Grids>, blocks, 256, 0, s, perm, b.cnt_sorted, b.off_sorted, rect_lo, rect_hi, N, cap, b.pair_tile[0], b.pair_val[0], stats, grids);
         note_launch();
         const int spar = radix_sort_pairs(b.pair_tile[0], b.pair_val[0], b.pair_tile[1], b.pair_val[1], b.n_sort + 1, 0, cap,
             kRectBits + int(higher_msb(n_super)), b.sort_tmp, n_sms, s, stats, kRectBits);
         if (int(higher_msb(n_super)) <= 8) {
-            k_super_plan<<<1, kSortBins, 0, s>>>(radix_digit_totals(b.sort_tmp, cap), n_super, b.super_ranges, b.chunk_base, b.n_sort);
+            launch_chained(k_super_plan, 1, kSortBins, 0, s, radix_digit_totals(b.sort_tmp, cap), n_super, b.super_ranges, b.chunk_base, b.n_sort);
         } else {
             const uint32_t want = (cap + 255) / 256, limit = uint32_t(n_sms) * 16;
             cudaMemsetAsync(b.super_ranges, 0, size_t(n_super) * 2 * sizeof(int32_t), s);
-            k_tile_ranges<<<want < limit ? want : limit, 256, 0, s>>>(b.pair_tile[spar], b.n_sort + 1, b.super_ranges, n_super, stats, kRectBits);
-            k_chunk_plan<<<1, 1024, 0, s>>>(b.super_ranges, n_super, b.chunk_base, b.n_sort);
+            launch_chained(k_tile_ranges, want < limit ? want : limit, 256, 0, s, b.pair_tile[spar], b.n_sort + 1, b.super_ranges, n_super, stats, kRectBits);
+            launch_chained(k_chunk_plan, 1, 1024, 0, s, b.super_ranges, n_super, b.chunk_base, b.n_sort);
             note_launch();
         }
         const ChunkRows rows = chunk_rows(b);
         const uint32_t cgrid = rows.max_chunks < uint32_t(n_sms) * 8 ? rows.max_chunks : uint32_t(n_sms) * 8;
-        k_chunk_counts<Grids><<<cgrid, kChunkThreads, 0, s>>>(b.pair_tile[spar], b.pair_val[spar], N, b.super_ranges, b.chunk_base, n_super, b.n_sort, rows,
+        launch_chained(k_chunk_counts<Grids>, cgrid, kChunkThreads, 0, s, b.pair_tile[spar], b.pair_val[spar], N, b.super_ranges, b.chunk_base, n_super, b.n_sort, rows,
             stats, grids);
-        k_chunk_prefix<Grids><<<n_super, kSuperTiles * kPrefixParts, 0, s>>>(b.chunk_base, n_super, rows, b.tile_total, n_tiles, stats, grids);
+        launch_chained(k_chunk_prefix<Grids>, n_super, kSuperTiles * kPrefixParts, 0, s, b.chunk_base, n_super, rows, b.tile_total, n_tiles, stats, grids);
         note_launch(3);
         if (n_tiles <= kScanSingleMax) {
-            k_scan_single<<<1, 1024, 0, s>>>(b.tile_total, n_tiles, b.tile_incl, ScanTotal { nullptr, 0u }, ranges, cap);
+            launch_chained(k_scan_single, 1, 1024, 0, s, b.tile_total, n_tiles, b.tile_incl, ScanTotal { nullptr, 0u }, ranges, cap);
             note_launch();
         } else {
             inclusive_scan_u32(b.tile_total, b.tile_incl, n_tiles, b.scan_tmp, s);
-            k_tile_ranges_from_counts<<<(n_tiles + 255) / 256, 256, 0, s>>>(b.tile_total, b.tile_incl, n_tiles, cap, ranges);
+            launch_chained(k_tile_ranges_from_counts, (n_tiles + 255) / 256, 256, 0, s, b.tile_total, b.tile_incl, n_tiles, cap, ranges);
             note_launch();
         }
         static bool smem_set = false; // one opt-in per instantiation, above the 48 KB default
@@ -883,7 +895,7 @@ inline int run_binning_grids(uint32_t N, uint32_t n_tiles, uint32_t n_super, con
             cudaFuncSetAttribute(k_chunk_emit<Grids>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(chunk_emit_smem()));
             smem_set = true;
         }
-        k_chunk_emit<Grids><<<cgrid, kChunkThreads, chunk_emit_smem(), s>>>(b.pair_tile[spar], b.pair_val[spar], N, b.super_ranges, b.chunk_base, n_super,
+        launch_chained(k_chunk_emit<Grids>, cgrid, kChunkThreads, chunk_emit_smem(), s, b.pair_tile[spar], b.pair_val[spar], N, b.super_ranges, b.chunk_base, n_super,
             b.n_sort, rows, b.tile_total, b.tile_incl, cap, b.pair_tile[1 - spar], b.pair_val[1 - spar], stats, grids);
         note_launch();
     } else {

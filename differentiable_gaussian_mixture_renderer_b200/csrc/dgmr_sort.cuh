@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "dgmr_chain.cuh"
 #include "dgmr_launch_count.h"
 
 namespace dgmr {
@@ -42,6 +43,7 @@ __device__ __forceinline__ uint32_t dev_count(const uint32_t* n_dev, uint32_t n_
 // per-tile sums of `in` (tile = kSortTile items)
 static __global__ void k_scan_tile_sums(const uint32_t* __restrict__ in, uint32_t n, uint32_t* __restrict__ tile_sums)
 {
+    chain_start();
     __shared__ uint32_t warp_sums[kSortWarps];
     const uint32_t tile = blockIdx.x;
     const uint32_t base = tile * kSortTile;
@@ -69,6 +71,7 @@ static __global__ void k_scan_tile_sums(const uint32_t* __restrict__ in, uint32_
 // exclusive scan of the tile sums in one block (tile counts are small)
 static __global__ void k_scan_tile_offsets(uint32_t* __restrict__ tile_sums, uint32_t n_tiles)
 {
+    chain_start();
     __shared__ uint32_t carry;
     __shared__ uint32_t warp_tot[32];
     if (threadIdx.x == 0)
@@ -148,6 +151,7 @@ template <bool kSums>
 static __global__ void __launch_bounds__(kSortThreads) k_scan_apply(const uint32_t* __restrict__ in, uint32_t n, const uint32_t* __restrict__ tile_offsets,
     uint32_t* __restrict__ out, ScanTotal total)
 {
+    chain_start();
     __shared__ uint32_t warp_tot[kSortWarps], warp_before[kSortWarps];
     const uint32_t tile = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -207,6 +211,7 @@ __device__ __forceinline__ bool pass_is_copy(const uint32_t* range, int shift)
 // min / max of the live keys into range (initialised to {~0, 0})
 static __global__ void k_key_range(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ live, uint32_t n, uint32_t* __restrict__ range)
 {
+    chain_start();
     uint32_t lo = 0xffffffffu, hi = 0u;
     // four items per thread and step, every load issued before the first is used
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -256,6 +261,7 @@ static __global__ void k_key_range(const uint32_t* __restrict__ keys, const uint
 static __global__ void k_radix_hist(uint32_t* __restrict__ keys, const uint32_t* n_dev, uint32_t n_static, uint32_t capacity, int shift, uint32_t mask,
     uint32_t* __restrict__ hist, uint32_t tile_stride, const uint32_t* __restrict__ range, const uint32_t* __restrict__ live, bool rebase)
 {
+    chain_start();
     __shared__ uint32_t h[kSortWarps][kSortBins];
     if (pass_is_copy(range, shift))
         return;
@@ -305,6 +311,7 @@ static __global__ void k_radix_hist(uint32_t* __restrict__ keys, const uint32_t*
 static __global__ void k_radix_scan_rows(uint32_t* __restrict__ hist, const uint32_t* n_dev, uint32_t n_static, uint32_t capacity, uint32_t tile_stride,
     uint32_t* __restrict__ digit_total, const uint32_t* __restrict__ range, int shift)
 {
+    chain_start();
     __shared__ uint32_t warp_tot[kSortWarps];
     __shared__ uint32_t carry;
     if (pass_is_copy(range, shift))
@@ -375,6 +382,7 @@ static __global__ void __launch_bounds__(256) k_radix_scatter(const uint32_t* __
     const uint32_t* __restrict__ hist, uint32_t tile_stride, const uint32_t* __restrict__ digit_total, uint32_t* __restrict__ stats,
     const uint32_t* __restrict__ range)
 {
+    chain_start();
     __shared__ uint32_t wcount[kSortWarps][kSortBins];
     __shared__ uint32_t gbase[kSortBins]; // global start of this tile's run of each digit
     __shared__ uint32_t lbase[kSortBins]; // start of each digit's run inside the tile
@@ -522,7 +530,7 @@ inline size_t radix_temp_bytes(uint32_t capacity)
 // by the first pass and passes over all-zero digits copy the values only; the
 // sorted keys are then not produced (only the values' order is).
 inline int radix_sort_pairs(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, const uint32_t* n_dev, uint32_t n_static, uint32_t capacity, int end_bit,
-    void* temp, int n_sms, cudaStream_t stream, uint32_t* stats = nullptr, int begin_bit = 0, const uint32_t* range = nullptr,
+    void* temp, int n_sms, const ChainStream& stream, uint32_t* stats = nullptr, int begin_bit = 0, const uint32_t* range = nullptr,
     const uint32_t* live = nullptr)
 {
     const uint32_t tiles = (capacity + kSortTile - 1) / kSortTile;
@@ -545,9 +553,9 @@ inline int radix_sort_pairs(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* 
         uint32_t* vi = cur ? v1 : v0;
         uint32_t* ko = cur ? k0 : k1;
         uint32_t* vo = cur ? v0 : v1;
-        k_radix_hist<<<grid, kSortThreads, 0, stream>>>(ki, n_dev, n_static, capacity, shift, mask, hist, stride, range, live, shift == begin_bit);
-        k_radix_scan_rows<<<kSortBins, kSortThreads, 0, stream>>>(hist, n_dev, n_static, capacity, stride, dtotal, range, shift);
-        k_radix_scatter<<<grid, kSortThreads, 0, stream>>>(ki, vi, ko, vo, n_dev, n_static, capacity, shift, mask, hist, stride, dtotal, stats, range);
+        launch_chained(k_radix_hist, grid, kSortThreads, 0, stream, ki, n_dev, n_static, capacity, shift, mask, hist, stride, range, live, shift == begin_bit);
+        launch_chained(k_radix_scan_rows, kSortBins, kSortThreads, 0, stream, hist, n_dev, n_static, capacity, stride, dtotal, range, shift);
+        launch_chained(k_radix_scatter, grid, kSortThreads, 0, stream, ki, vi, ko, vo, n_dev, n_static, capacity, shift, mask, hist, stride, dtotal, stats, range);
         note_launch(3);
         cur ^= 1;
     }
@@ -563,6 +571,7 @@ constexpr uint32_t kScanSingleMax = 32u * 1024u;
 static __global__ void __launch_bounds__(1024) k_scan_single(const uint32_t* __restrict__ in, uint32_t n, uint32_t* __restrict__ out, ScanTotal total,
     int32_t* __restrict__ ranges, uint32_t range_cap)
 {
+    chain_start();
     __shared__ uint32_t warp_tot[2][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t carry = 0;
@@ -612,25 +621,25 @@ inline size_t scan_temp_bytes(uint32_t n) { return ((size_t(n) + kSortTile - 1) 
 // block can sum the tiles before it, else three
 constexpr uint32_t kScanOneBlock = 16u * 1024u;
 static_assert(kScanOneBlock <= kScanSingleMax, "the one-block scan's limit");
-inline void inclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, void* temp, cudaStream_t stream, ScanTotal total = { nullptr, 0u })
+inline void inclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, void* temp, const ChainStream& stream, ScanTotal total = { nullptr, 0u })
 {
     if (n == 0)
         return;
     if (n <= kScanOneBlock) {
-        k_scan_single<<<1, 1024, 0, stream>>>(in, n, out, total, nullptr, 0u);
+        launch_chained(k_scan_single, 1, 1024, 0, stream, in, n, out, total, nullptr, 0u);
         note_launch();
         return;
     }
     const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
     uint32_t* sums = static_cast<uint32_t*>(temp);
-    k_scan_tile_sums<<<tiles, kSortThreads, 0, stream>>>(in, n, sums);
+    launch_chained(k_scan_tile_sums, tiles, kSortThreads, 0, stream, in, n, sums);
     if (tiles <= kScanOwnSums) {
-        k_scan_apply<true><<<tiles, kSortThreads, 0, stream>>>(in, n, sums, out, total);
+        launch_chained(k_scan_apply<true>, tiles, kSortThreads, 0, stream, in, n, sums, out, total);
         note_launch(2);
         return;
     }
-    k_scan_tile_offsets<<<1, 1024, 0, stream>>>(sums, tiles);
-    k_scan_apply<false><<<tiles, kSortThreads, 0, stream>>>(in, n, sums, out, total);
+    launch_chained(k_scan_tile_offsets, 1, 1024, 0, stream, sums, tiles);
+    launch_chained(k_scan_apply<false>, tiles, kSortThreads, 0, stream, in, n, sums, out, total);
     note_launch(3);
 }
 

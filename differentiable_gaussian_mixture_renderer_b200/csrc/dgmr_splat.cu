@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(kTilePixels, 5) k_splat_blend_tiles(const int3
     const float4* __restrict__ rec, const float* __restrict__ rgb, uint32_t N, uint32_t cap, uint32_t* __restrict__ stats,
     const uint32_t* __restrict__ tile_order, const __grid_constant__ Frames frames)
 {
+    chain_start();
     constexpr int kThreads = kTilePixels;
     constexpr int kBatch = kThreads;
     constexpr int kWarps = kThreads / 32;
@@ -498,6 +499,7 @@ __global__ void __launch_bounds__(kQuarterWarps * 32, 5) k_splat_blend_quarters(
     const float4* __restrict__ rec, const float* __restrict__ rgb, uint32_t N, uint32_t cap, uint32_t* __restrict__ stats,
     const uint32_t* __restrict__ tile_order, const __grid_constant__ Frames frames)
 {
+    chain_start();
     constexpr int kGroup = 4;
     __shared__ float4 s_r0[kQuarterWarps][32];
     __shared__ float4 s_r1[kQuarterWarps][32]; // (2b, opacity, q_cut, 1-based list index as int bits)
@@ -636,9 +638,9 @@ void launch_blend(int side, uint32_t n_tiles, const int32_t* ranges, const uint3
     if (n_tiles == 0)
         return;
     if (side == 8)
-        k_splat_blend_quarters<Frames><<<n_tiles, kQuarterWarps * 32, 0, s>>>(ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
+        launch_chained(k_splat_blend_quarters<Frames>, n_tiles, kQuarterWarps * 32, 0, ChainStream(s, n_tiles <= kChainBlendTiles), ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
     else
-        k_splat_blend_tiles<Frames><<<n_tiles, kTilePixels, 0, s>>>(ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
+        launch_chained(k_splat_blend_tiles<Frames>, n_tiles, kTilePixels, 0, ChainStream(s, n_tiles <= kChainBlendTiles), ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
     note_launch();
 }
 
@@ -1114,6 +1116,7 @@ __global__ void __launch_bounds__(kOrderWarps * 32) k_blend_tile_order(const int
     const float4* __restrict__ rec, uint32_t N, uint32_t cap, uint32_t n_tiles, uint32_t* __restrict__ bucket, uint32_t* __restrict__ blocks_done,
     uint32_t* __restrict__ order, const __grid_constant__ Frames frames)
 {
+    chain_start();
     constexpr int kSample = 128;
     __shared__ uint32_t count[kCostBuckets];
     __shared__ uint32_t cursor[kCostBuckets];
@@ -1257,7 +1260,8 @@ void launch_tile_order(const SplatLayout& L, int par, uint32_t N, uint32_t cap, 
 {
     if (n_tiles == 0)
         return;
-    k_blend_tile_order<Frames><<<(n_tiles + kOrderWarps - 1) / kOrderWarps, kOrderWarps * 32, 0, s>>>(L.ranges, L.bin.pair_val[par], L.blend_rec, N, cap,
+    launch_chained(k_blend_tile_order<Frames>, (n_tiles + kOrderWarps - 1) / kOrderWarps, kOrderWarps * 32, 0,
+        ChainStream(s, n_tiles <= kChainBlendTiles), L.ranges, L.bin.pair_val[par], L.blend_rec, N, cap,
         n_tiles, L.tile_cost, L.bin.n_sort + 6, L.tile_order, frames);
     note_launch();
 }
@@ -1333,7 +1337,7 @@ dgmr_status dgmr_splat_preprocess(const dgmr_scene* scene, const dgmr_camera* ca
     uint32_t* st_dev = stats ? reinterpret_cast<uint32_t*>(stats) : L.stats;
     launch_preprocess(scene, cam, L, st_dev, s);
     if (scene->n_gaussians > 0) {
-        k_pair_count<<<1, 1, 0, s>>>(L.point_offsets, uint32_t(scene->n_gaussians), 0xffffffffu, st_dev, L.bin.n_sort);
+        launch_chained(k_pair_count, 1, 1, 0, s, L.point_offsets, uint32_t(scene->n_gaussians), 0xffffffffu, st_dev, L.bin.n_sort);
         note_launch();
     }
     return launch_status();
@@ -1556,7 +1560,7 @@ void batch_preprocess(const BatchPlan& plan, uint32_t* st_dev, cudaStream_t s)
         return;
     k_batch_preprocess<<<(G + 255) / 256, 256, 0, s>>>(batch_pre(L, G), plan.tab);
     note_launch();
-    inclusive_scan_u32(L.tiles_touched, L.point_offsets, G, L.bin.scan_tmp, s);
+    inclusive_scan_u32(L.tiles_touched, L.point_offsets, G, L.bin.scan_tmp, ChainStream(s, G <= kChainMost));
 }
 
 } // namespace
@@ -1591,7 +1595,7 @@ dgmr_status dgmr_splat_batch_preprocess(const dgmr_scene* scenes, int32_t n_scen
     uint32_t* st_dev = stats ? reinterpret_cast<uint32_t*>(stats) : plan.L.stats;
     batch_preprocess(plan, st_dev, s);
     if (plan.tab.G > 0) {
-        k_pair_count<<<1, 1, 0, s>>>(plan.L.point_offsets, plan.tab.G, 0xffffffffu, st_dev, plan.L.bin.n_sort);
+        launch_chained(k_pair_count, 1, 1, 0, s, plan.L.point_offsets, plan.tab.G, 0xffffffffu, st_dev, plan.L.bin.n_sort);
         note_launch();
     }
     return launch_status();
