@@ -15,6 +15,7 @@ namespace dgmr {
 
 // per-Gaussian backward accumulators (double): mass, rgb(3), inverse covariance(6), centroid(3)
 constexpr unsigned kVmAcc = 13;
+constexpr unsigned kMarchRec = 5; // 16-byte words of a march record
 
 template <class T>
 struct ConstSamplesT {
@@ -43,6 +44,7 @@ struct VmLayout {
     uint32_t* stats;
     uint32_t* pre_scan_tmp;
     double* acc; // backward, [N,13]: mass, rgb(3), inverse covariance(6), centroid(3)
+    float4* rec; // float only, [N,5]: the march's records (k_vm_records)
     BinningBuffers bin;
     size_t pre_bytes;
     size_t bytes;
@@ -63,6 +65,7 @@ inline VmLayout<T> vm_layout(uint32_t N, uint32_t n_tiles, uint32_t cap, void* b
     L.pre_scan_tmp = c.take<uint32_t>(scan_temp_bytes(N) / 4 + 8); // + room for k_pair_count's eight counters
     L.pre_bytes = c.off;
     L.acc = c.take<double>(size_t(N) * kVmAcc);
+    L.rec = c.take<float4>(sizeof(T) == 4 ? size_t(N) * kMarchRec : 0);
     carve_binning(c, L.bin, N, n_tiles, cap);
     L.bytes = c.off;
     return L;
@@ -207,6 +210,44 @@ __device__ __forceinline__ V3<T> pixel_dir(const CameraT<T>& cam, unsigned px, u
     return mul3(d, il);
 }
 
+// What the float march reads of a Gaussian, 5 x 16 bytes:
+//   Q00 Q01 Q02 Q11 | Q12 Q22 mass depth | centre, 0 | Qc, c'Qc | log, t, 0, 0
+// with Q the inverse filtered covariance, c = centre - camera, log the base-2
+// logarithm of mass sqrt(det Q) / 2 pi and t = tr Q |c|^2 (ray_may_use).  log is
+// +inf, so that nothing is turned away by it, where Q is not clearly positive
+// definite or a value is out of the range the bounds there are for.
+__device__ __forceinline__ void write_march_record(float4* rec, size_t i, V3<float> mu, const float* inv_cov, float mass, float depth, V3<float> o)
+{
+    S3<float> Q;
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        Q.v[k] = inv_cov[k];
+    const V3<float> c = sub3(mu, o);
+    const V3<float> Qc = { (Q.v[0] * c.x + Q.v[1] * c.y) + Q.v[2] * c.z, (Q.v[1] * c.x + Q.v[3] * c.y) + Q.v[4] * c.z, (Q.v[2] * c.x + Q.v[4] * c.y) + Q.v[5] * c.z };
+    const float det = det_sym3(Q), tr = (Q.v[0] + Q.v[3]) + Q.v[5], cc = dot3(c, c);
+    const float d0 = Q.v[0], d1 = Q.v[3], d2 = Q.v[5];
+    constexpr float kSure = 1.0e-4f;
+    const bool sure = d0 > 0.f && d1 > 0.f && d2 > 0.f && d0 * d1 - Q.v[1] * Q.v[1] > kSure * (d0 * d1) && d0 * d2 - Q.v[2] * Q.v[2] > kSure * (d0 * d2)
+        && d1 * d2 - Q.v[4] * Q.v[4] > kSure * (d1 * d2) && det > kSure * ((d0 * d1) * d2) && det > 1.0e-30f && tr < 1.0e9f && cc < 1.0e9f && mass > 1.0e-30f
+        && mass < 1.0e30f;
+    const float log_mass = sure ? __log2f(mass) + 0.5f * __log2f(det) - 2.6514961f : 1.f / 0.f;
+    rec += kMarchRec * i;
+    rec[0] = make_float4(Q.v[0], Q.v[1], Q.v[2], Q.v[3]);
+    rec[1] = make_float4(Q.v[4], Q.v[5], mass, depth);
+    rec[2] = make_float4(mu.x, mu.y, mu.z, 0.f);
+    rec[3] = make_float4(Qc.x, Qc.y, Qc.z, dot3(c, Qc));
+    rec[4] = make_float4(log_mass, tr * cc, 0.f, 0.f);
+}
+
+__global__ void __launch_bounds__(256) k_vm_records(const float* __restrict__ centroids, const float* __restrict__ inv_cov, const float* __restrict__ masses,
+    const float* __restrict__ depths, uint32_t N, V3<float> o, float4* __restrict__ rec)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < N)
+        write_march_record(rec, i, V3<float> { centroids[3 * size_t(i)], centroids[3 * size_t(i) + 1], centroids[3 * size_t(i) + 2] }, inv_cov + 6 * size_t(i),
+            masses[i], depths[i], o);
+}
+
 template <class T>
 struct VmMarch {
     const int32_t* ranges;
@@ -216,6 +257,7 @@ struct VmMarch {
     const T* masses;
     const T* rgb;
     const T* depths;
+    const float4* rec; // float: the records (k_vm_records) in place of the four arrays above but rgb
     T* fb;
     T* remaining_T;
     const T* grad_fb; // backward only
@@ -477,6 +519,17 @@ dgmr_status vm_preprocess(const dgmr_scene* scene, const dgmr_camera* camera, dg
     return launch_status();
 }
 
+// The march's records of a frame, float only.
+inline void launch_records(VmMarch<float>& a, const CameraT<float>& cam, uint32_t N, float4* rec, cudaStream_t s)
+{
+    a.rec = rec;
+    if (N == 0)
+        return;
+    k_vm_records<<<(N + 255) / 256, 256, 0, s>>>(a.centroids, a.inv_cov, a.masses, a.depths, N, V3<float> { cam.campos[0], cam.campos[1], cam.campos[2] }, rec);
+    note_launch();
+}
+inline void launch_records(VmMarch<double>&, const CameraT<double>&, uint32_t, float4*, cudaStream_t) { }
+
 template <class T>
 dgmr_status vm_render(const dgmr_scene* scene, const dgmr_camera* camera, dgmr_vm_cache* c, int64_t cap64, void* workspace, size_t workspace_bytes,
     dgmr_frame_stats* stats, cudaStream_t s, const dgmr_render_options* options, void* store = nullptr, uint32_t store_steps = 0)
@@ -517,6 +570,7 @@ dgmr_status vm_render(const dgmr_scene* scene, const dgmr_camera* camera, dgmr_v
         carve_step_store<T>(store, uint32_t(camera->width) * uint32_t(camera->height), store_steps, &a.store_borders, &a.store_sections);
         a.store_steps = store_steps;
     }
+    launch_records(a, cam, N, L.rec, s);
     const uint32_t* order = march_order(c->i_ranges, cam, workspace, L.bytes, workspace_bytes, s);
     k_vm_march_warp<T, VmSingleFrame<T>><<<cam.gx * cam.gy * (kTilePixels / kRayWarps), kRayWarps * 32, 0, s>>>(a, VmSingleFrame<T> { cam }, order);
     note_launch();
@@ -556,6 +610,7 @@ dgmr_status vm_backward(const dgmr_scene* scene, const dgmr_camera* camera, cons
             &a.store_sections);
         a.store_steps = store_steps;
     }
+    launch_records(a, cam, N, L.rec, s);
     const uint32_t* order = march_order(c->i_ranges, cam, workspace, L.bytes, workspace_bytes, s);
     k_vm_march_warp_bwd<T, VmSingleFrame<T>><<<cam.gx * cam.gy * (kTilePixels / kRayWarps), kRayWarps * 32, 0, s>>>(a, VmSingleFrame<T> { cam }, order);
     note_launch();
@@ -606,8 +661,8 @@ struct VmBatchFrames {
 };
 
 // Frame workspace: statistics, the per-slot arrays (the single frame's cache,
-// plus a copy of each slot's centroid so the march reads every list entry by
-// its slot), the backward's accumulators, ranges, remaining transmittance of
+// and each slot's march record, by which the march reads every list entry),
+// the backward's accumulators, ranges, remaining transmittance of
 // every pixel, the march order and the binning's Gaussian-sized buffers.
 // Pair workspace: the binning's pair buffers and sort scratch.
 struct VmBatchLayout {
@@ -621,7 +676,7 @@ struct VmBatchLayout {
     float* masses;
     uint32_t* tiles_touched;
     uint32_t* point_offsets;
-    float* centroids;
+    float4* rec; // [G,5] the march's records
     double* acc;
     int32_t* ranges;
     float* remaining_T;
@@ -646,7 +701,7 @@ inline VmBatchLayout vm_batch_layout(uint32_t G, uint32_t n_tiles, size_t n_px, 
     L.masses = c.take<float>(G);
     L.tiles_touched = c.take<uint32_t>(G);
     L.point_offsets = c.take<uint32_t>(G);
-    L.centroids = c.take<float>(size_t(G) * 3);
+    L.rec = c.take<float4>(size_t(G) * kMarchRec);
     L.acc = c.take<double>(size_t(G) * kVmAcc);
     L.ranges = c.take<int32_t>(size_t(n_tiles) * 2);
     L.remaining_T = c.take<float>(n_px);
@@ -661,8 +716,8 @@ inline VmBatchLayout vm_batch_layout(uint32_t G, uint32_t n_tiles, size_t n_px, 
 }
 
 // One thread per (view, Gaussian) slot: the single frame's preprocess with the
-// view's camera, then the slot's depth key, identity permutation and centroid.
-__global__ void __launch_bounds__(128) k_vm_batch_preprocess(VmPre<float> out, float* __restrict__ slot_centroids, uint32_t* __restrict__ depth_key,
+// view's camera, then the slot's depth key, identity permutation and march record.
+__global__ void __launch_bounds__(128) k_vm_batch_preprocess(VmPre<float> out, float4* __restrict__ rec, uint32_t* __restrict__ depth_key,
     uint32_t* __restrict__ perm, const __grid_constant__ BatchTable tab)
 {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -686,9 +741,9 @@ __global__ void __launch_bounds__(128) k_vm_batch_preprocess(VmPre<float> out, f
     vm_preprocess_one(p, bv.cam, i, g);
     depth_key[g] = __float_as_uint(p.depths[g]);
     perm[g] = g;
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        slot_centroids[3 * size_t(g) + k] = sc.centroids[3 * size_t(i) + k];
+    const float* mu = sc.centroids + 3 * size_t(i);
+    write_march_record(rec, g, V3<float> { mu[0], mu[1], mu[2] }, p.inv_cov + 6 * size_t(g), p.masses[g], p.depths[g],
+        V3<float> { bv.cam.campos[0], bv.cam.campos[1], bv.cam.campos[2] });
 }
 
 // per scene Gaussian: zero its gradient rows, then add the chain rule of every
@@ -777,7 +832,7 @@ void vm_batch_preprocess(const VmBatchPlan& plan, uint32_t* st_dev, cudaStream_t
         return;
     VmPre<float> p { G, nullptr, nullptr, 1, 0, nullptr, nullptr, nullptr, L.rects, L.rgb, L.clamped, L.depths, L.xy, L.inv_cov, L.masses,
         L.tiles_touched, 0.f, Formulation::Opacity };
-    k_vm_batch_preprocess<<<(G + 127) / 128, 128, 0, s>>>(p, L.centroids, L.bin.depth_key, L.bin.perm, plan.tab);
+    k_vm_batch_preprocess<<<(G + 127) / 128, 128, 0, s>>>(p, L.rec, L.bin.depth_key, L.bin.perm, plan.tab);
     note_launch();
     inclusive_scan_u32(L.tiles_touched, L.point_offsets, G, L.bin.scan_tmp, ChainStream(s, G <= kChainMost));
 }
@@ -788,11 +843,8 @@ VmMarch<float> vm_batch_march(const VmBatchLayout& L, const uint32_t* list, uint
     VmMarch<float> a {};
     a.ranges = L.ranges;
     a.list = reinterpret_cast<const int32_t*>(list);
-    a.centroids = L.centroids;
-    a.inv_cov = L.inv_cov;
-    a.masses = L.masses;
+    a.rec = L.rec;
     a.rgb = L.rgb;
-    a.depths = L.depths;
     a.stats = st_dev;
     a.cs = const_samples<float>();
     a.mode = DGMR_RENDER_FULL;

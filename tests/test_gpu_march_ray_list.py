@@ -52,3 +52,23 @@ def test_tile_list_longer_than_16_bit_offsets(cuda):
     rng = np.random.default_rng(9)
     sc.weights = np.where(rng.random(n) < 0.01, rng.uniform(0.2, 0.9, size=n), 1e-4).astype(np.float32)
     assert check(sc, S.make_camera(16, 16), cuda, torch.float32) > 65_536
+
+
+@pytest.mark.parametrize("n,extent,scales,eye,size", [
+    (3000, 1.0, (0.0005, 0.5), (0.0, 0.0, -3.0), (40, 24)),  # needles and plates, 1000 to 1
+    (2000, 0.5, (0.005, 0.05), (0.1, 0.0, -0.3), (24, 24)),  # from inside the cloud
+    (3000, 30.0, (0.2, 2.0), (3.0, 1.0, -60.0), (32, 32)),  # far away
+    (20000, 1.0, (0.005, 0.05), (0.0, 0.0, -2.5), (16, 16)),  # many candidates per ray, most turned away
+])
+def test_entries_turned_away_are_not_usable(cuda, n, extent, scales, eye, size):
+    """The approximate test on a Gaussian's record turns away no entry that the
+    exact one would use: the march fills as many bins as the oracle."""
+    sc = S.make_scene(n, seed=n, extent=extent, scale_range=scales)
+    cam = S.make_camera(*size, eye=eye)
+    with O.decision_audit() as audit:
+        O.vm_forward(sc, cam)
+    counter = torch.zeros(1, dtype=torch.int64, device=cuda)
+    cache, ts = run_vm(sc, cam, cuda, torch.float32)
+    cpp_binding.forward(*ts, cam.width, cam.height, cam.tan_fovx, cam.tan_fovy, sc.sh_degree, work_counter=counter)
+    assert int(counter.item()) == audit["fills"] > 0
+    check(sc, cam, cuda, torch.float32)
