@@ -448,17 +448,17 @@ __device__ __forceinline__ V3<T> sh_to_colour(const T* sh, uint32_t i, int strid
     return { max_f(r.x, T(0)), max_f(r.y, T(0)), max_f(r.z, T(0)) };
 }
 
-// grad/math.h:203-282.  Writes d/dsh for the first `stride` coefficients
-// (those beyond the caller's stride are padded with `pad` and dropped, like the
-// reference's cat + slice) and returns d/ddirection.
+// grad/math.h:203-282.  Writes d/dsh for the first `stride` coefficients to the
+// Gaussian's row (those beyond the caller's stride are padded with `pad` and
+// dropped, like the reference's cat + slice) and returns d/ddirection.
 template <class T>
 __device__ __forceinline__ V3<T> grad_sh_to_colour(const T* sh, uint32_t i, int stride, int deg, V3<T> dir, V3<T> g_in, const uint8_t* mask, T pad,
-    T* g_sh_out, bool accumulate = false)
+    T* g_row, bool accumulate = false)
 {
     const V3<T> g = { mask[0] ? g_in.x : T(0), mask[1] ? g_in.y : T(0), mask[2] ? g_in.z : T(0) };
     const auto put = [&](int j, T basis) {
         if (j < stride) {
-            T* p = g_sh_out + (size_t(i) * stride + j) * 3;
+            T* p = g_row + 3 * j;
             if (accumulate) {
                 p[0] += g.x * basis;
                 p[1] += g.y * basis;
@@ -473,7 +473,7 @@ __device__ __forceinline__ V3<T> grad_sh_to_colour(const T* sh, uint32_t i, int 
     const auto S = [&](int j) { return sh_load(sh, i, stride, j, pad); };
     if (!accumulate) {
         for (int j = 0; j < stride; ++j) {
-            T* p = g_sh_out + (size_t(i) * stride + j) * 3;
+            T* p = g_row + 3 * j;
             p[0] = p[1] = p[2] = T(0);
         }
     }

@@ -403,7 +403,7 @@ __device__ __forceinline__ void vm_bwd_gaussian_one(const VmBwdGauss<T>& p, cons
     }
     const V3<T> dir = { delta.x / dist, delta.y / dist, delta.z / dist };
     const V3<T> g_dir = grad_sh_to_colour(p.sh, i, p.sh_stride, p.sh_degree, dir, V3<T> { T(a[1]), T(a[2]), T(a[3]) }, p.clamped + 3 * size_t(o), T(1),
-        p.g_sh, kAdd);
+        p.g_sh + size_t(i) * 3 * p.sh_stride, kAdd);
     V3<T> g_mu = mul3(g_dir, T(1) / dist);
     T g_dist = -dot3(g_dir, delta) / (dist * dist);
     S3<T> g_inv;

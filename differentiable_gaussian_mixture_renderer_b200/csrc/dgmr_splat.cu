@@ -983,21 +983,43 @@ __device__ __forceinline__ void store_gaussian_grads(const SplatBwdGauss& p, uin
         p.g_rotations[4 * size_t(i) + k] = g.q[k];
 }
 
-__device__ __forceinline__ void zero_sh_grads(const SplatBwdGauss& p, uint32_t i)
+// A block's SH gradient rows in shared memory, one per thread, an odd number of
+// words apart (no bank conflicts); each warp copies its 32 rows out together.
+// Stored by each thread, a row of 16 coefficients is 48 stores that touch 32
+// sectors each, twice with the zeros that go first.  The kernel at 1M with 1, 4, 9
+// and 16 coefficients: 80, 126, 295, 632 us direct; 88, 103, 134, 319 through rows.
+// So rows of one coefficient (kShDirect) are stored directly; a batch, which adds
+// up several views' rows, always goes through shared memory.
+constexpr int kBwdGaussThreads = 128;
+constexpr int kShDirect = 1;
+__host__ __device__ constexpr int sh_row_words(int sh_stride) { return 3 * sh_stride | 1; }
+
+__device__ __forceinline__ void store_sh_rows(const SplatBwdGauss& p, const float* rows, uint32_t i0, uint32_t n_rows, int lane, int step)
 {
-    for (int k = 0; k < p.sh_stride * 3; ++k)
-        p.g_sh[size_t(i) * p.sh_stride * 3 + k] = 0.f;
+    const int width = 3 * p.sh_stride;
+    float* out = p.g_sh + size_t(i0) * width;
+    int r = 0, c = lane;
+    __syncwarp();
+    for (uint32_t t = uint32_t(lane); t < n_rows * uint32_t(width); t += 32) {
+        while (c >= width) {
+            c -= width;
+            ++r;
+        }
+        out[t] = rows[r * step + c];
+        c += 32;
+    }
 }
 
 // per-Gaussian chain rule: conic -> 2-D covariance -> projection adjoint, SH.
 // Gaussian i of the scene, per-view state at slot o, on a tile of its view; the
-// result is added to `sum` and, for the SH coefficients, written to their
-// gradient rows (kAddSh: added to them), so several views of one scene sum up.
+// result is added to `sum` and, for the SH coefficients, written to the Gaussian's
+// `row` (kAddSh: added to it), so several views of one scene sum up.
 // Rows and sums are stored once per Gaussian (zeroed first and added to in
-// memory, with the same arithmetic: 106.6 us at 1M, SH degree 0, now 85.9; bound by
-// its ~1700 instructions per warp, 29 us of memory traffic).
+// memory, with the same arithmetic: 106.6 us at 1M, SH degree 0, now 85.9, and 78
+// with 80 registers instead of 96; bound by its ~1900 instructions per warp, 29
+// us of memory traffic).
 template <bool kAddSh>
-__device__ __forceinline__ void bwd_gaussian_one(const SplatBwdGauss& p, const CameraT<float>& cam, uint32_t i, uint32_t o, GaussianGrads& sum)
+__device__ __forceinline__ void bwd_gaussian_one(const SplatBwdGauss& p, const CameraT<float>& cam, uint32_t i, uint32_t o, GaussianGrads& sum, float* row)
 {
     double m[9];
 #pragma unroll
@@ -1030,7 +1052,7 @@ __device__ __forceinline__ void bwd_gaussian_one(const SplatBwdGauss& p, const C
     const float vl = dgmr_fm::sqrt_f(dot3(v, v));
     const V3<float> dir = mul3(v, 1.f / vl);
     const V3<float> g_dir
-        = grad_sh_to_colour(p.sh, i, p.sh_stride, p.sh_degree, dir, V3<float> { a[6], a[7], a[8] }, p.clamped + 3 * size_t(o), 0.f, p.g_sh, kAddSh);
+        = grad_sh_to_colour(p.sh, i, p.sh_stride, p.sh_degree, dir, V3<float> { a[6], a[7], a[8] }, p.clamped + 3 * size_t(o), 0.f, row, kAddSh);
     const float gd = dot3(g_dir, dir);
     g_mu = add3(g_mu, mul3(sub3(g_dir, mul3(dir, gd)), 1.f / vl));
     sum.weight += g_weight;
@@ -1043,17 +1065,27 @@ __device__ __forceinline__ void bwd_gaussian_one(const SplatBwdGauss& p, const C
         sum.q[k] += g_q[k];
 }
 
-__global__ void __launch_bounds__(128) k_splat_bwd_gaussians(SplatBwdGauss p, CameraT<float> cam)
+// kRows: through shared memory (store_sh_rows), else each thread stores its row.
+template <bool kRows>
+__global__ void __launch_bounds__(kBwdGaussThreads, 6) k_splat_bwd_gaussians(SplatBwdGauss p, CameraT<float> cam)
 {
+    extern __shared__ float sh_rows[];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.N)
-        return;
-    GaussianGrads g;
-    if (p.tiles_touched[i] != 0)
-        bwd_gaussian_one<false>(p, cam, i, i, g);
-    else
-        zero_sh_grads(p, i);
-    store_gaussian_grads(p, i, g);
+    const int spacing = sh_row_words(p.sh_stride);
+    if (i < p.N) {
+        float* row = kRows ? sh_rows + threadIdx.x * spacing : p.g_sh + size_t(i) * 3 * p.sh_stride;
+        GaussianGrads g;
+        if (p.tiles_touched[i] != 0) {
+            bwd_gaussian_one<false>(p, cam, i, i, g, row);
+        } else {
+            for (int k = 0; k < 3 * p.sh_stride; ++k)
+                row[k] = 0.f;
+        }
+        store_gaussian_grads(p, i, g);
+    }
+    const uint32_t i0 = i & ~31u;
+    if (kRows && i0 < p.N)
+        store_sh_rows(p, sh_rows + (threadIdx.x & ~31u) * spacing, i0, min(32u, p.N - i0), int(threadIdx.x & 31u), spacing);
 }
 
 } // namespace dgmr
@@ -1427,7 +1459,11 @@ dgmr_status dgmr_splat_backward(const dgmr_scene* scene, const dgmr_camera* came
     SplatBwdGauss p { N, static_cast<const float*>(scene->centroids), static_cast<const float*>(scene->sh), scene->sh_stride, scene->sh_degree,
         static_cast<const float*>(scene->weights), static_cast<const float*>(scene->scales), static_cast<const float*>(scene->rotations), L.clamped,
         L.tiles_touched, L.grad_acc, grad_sh, grad_weights, grad_centroids, grad_scales, grad_rotations, scene_formulation(scene, Formulation::Ots) };
-    k_splat_bwd_gaussians<<<(N + 127) / 128, 128, 0, s>>>(p, cam);
+    const uint32_t blocks = (N + kBwdGaussThreads - 1) / kBwdGaussThreads;
+    if (p.sh_stride > kShDirect)
+        k_splat_bwd_gaussians<true><<<blocks, kBwdGaussThreads, size_t(kBwdGaussThreads) * sh_row_words(p.sh_stride) * sizeof(float), s>>>(p, cam);
+    else
+        k_splat_bwd_gaussians<false><<<blocks, kBwdGaussThreads, 0, s>>>(p, cam);
     note_launch(2);
     return launch_status();
 }
@@ -1462,16 +1498,15 @@ __global__ void __launch_bounds__(256) k_batch_preprocess(SplatPre out, const __
 
 // per scene Gaussian: the chain rule of every view of its scene, added in view
 // order (deterministic, no atomics)
-__global__ void __launch_bounds__(128) k_batch_bwd_gaussians(SplatBwdGauss state, const __grid_constant__ BatchTable tab)
+__global__ void __launch_bounds__(kBwdGaussThreads, 6) k_batch_bwd_gaussians(SplatBwdGauss state, const __grid_constant__ BatchTable tab)
 {
+    extern __shared__ float sh_rows[];
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= tab.scene_off[tab.n_scenes])
-        return;
-    const uint32_t s = BatchTable::owner(tab.scene_off, tab.n_scenes, k);
+    const uint32_t total = tab.scene_off[tab.n_scenes];
+    const bool in = k < total;
+    const uint32_t s = BatchTable::owner(tab.scene_off, tab.n_scenes, in ? k : total - 1u);
     const BatchScene& sc = tab.scenes[s];
     const uint32_t i = k - tab.scene_off[s];
-    if (!sc.g_sh) // a scene entry without gradient outputs
-        return;
     SplatBwdGauss p = state;
     p.N = sc.n;
     p.centroids = sc.centroids;
@@ -1487,15 +1522,32 @@ __global__ void __launch_bounds__(128) k_batch_bwd_gaussians(SplatBwdGauss state
     p.g_scales = sc.g_scales;
     p.g_rotations = sc.g_rotations;
     p.form = sc.form;
-    zero_sh_grads(p, i);
-    GaussianGrads g;
-    for (uint32_t q = sc.view_begin; q < sc.view_end; ++q) {
-        const uint32_t v = tab.view_by_scene[q];
-        const uint32_t o = tab.g_off[v] + i;
-        if (tab.views[v].grad_fb && p.tiles_touched[o] != 0)
-            bwd_gaussian_one<true>(p, tab.views[v].cam, i, o, g);
+    // state.sh_stride: the largest of the scenes, by which the threads' rows are spaced
+    const int spacing = sh_row_words(state.sh_stride);
+    float* row = sh_rows + threadIdx.x * spacing;
+    const bool wanted = in && sc.g_sh; // a scene entry may have no gradient outputs
+    if (wanted) {
+        for (int c = 0; c < 3 * p.sh_stride; ++c)
+            row[c] = 0.f;
+        GaussianGrads g;
+        for (uint32_t q = sc.view_begin; q < sc.view_end; ++q) {
+            const uint32_t v = tab.view_by_scene[q];
+            const uint32_t o = tab.g_off[v] + i;
+            if (tab.views[v].grad_fb && p.tiles_touched[o] != 0)
+                bwd_gaussian_one<true>(p, tab.views[v].cam, i, o, g, row);
+        }
+        store_gaussian_grads(p, i, g);
     }
-    store_gaussian_grads(p, i, g);
+    // a warp of one scene copies its rows out together; where two scenes meet, every lane its own
+    const uint32_t there = __ballot_sync(0xffffffffu, in), want = __ballot_sync(0xffffffffu, wanted);
+    const uint32_t first_scene = __shfl_sync(0xffffffffu, s, 0), first_row = __shfl_sync(0xffffffffu, i, 0);
+    if (__all_sync(0xffffffffu, !in || s == first_scene)) {
+        if (want)
+            store_sh_rows(p, sh_rows + (threadIdx.x & ~31u) * spacing, first_row, uint32_t(__popc(there)), int(threadIdx.x & 31u), spacing);
+    } else if (wanted) {
+        for (int c = 0; c < 3 * p.sh_stride; ++c)
+            p.g_sh[size_t(i) * 3 * p.sh_stride + c] = row[c];
+    }
 }
 
 } // namespace dgmr
@@ -1649,9 +1701,13 @@ dgmr_status dgmr_splat_batch_backward(const dgmr_scene* scenes, int32_t n_scenes
     const int par = tile_sort_parity(plan.tab.n_stiles);
     cudaMemsetAsync(L.grad_acc, 0, size_t(G) * 9 * sizeof(double), s);
     launch_blend_bwd(plan.tab.n_tiles, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, G, L.grad_acc, L.tile_order, plan.tab, s);
-    SplatBwdGauss state { 0, nullptr, nullptr, 1, 0, nullptr, nullptr, nullptr, L.clamped, L.tiles_touched, L.grad_acc, nullptr, nullptr, nullptr, nullptr,
+    int sh_stride = 1;
+    for (int32_t k = 0; k < n_scenes; ++k)
+        sh_stride = scenes[k].sh_stride > sh_stride ? scenes[k].sh_stride : sh_stride;
+    SplatBwdGauss state { 0, nullptr, nullptr, sh_stride, 0, nullptr, nullptr, nullptr, L.clamped, L.tiles_touched, L.grad_acc, nullptr, nullptr, nullptr, nullptr,
         nullptr, Formulation::Ots };
-    k_batch_bwd_gaussians<<<(n_scene_gaussians + 127) / 128, 128, 0, s>>>(state, plan.tab);
+    k_batch_bwd_gaussians<<<(n_scene_gaussians + kBwdGaussThreads - 1) / kBwdGaussThreads, kBwdGaussThreads,
+        size_t(kBwdGaussThreads) * sh_row_words(sh_stride) * sizeof(float), s>>>(state, plan.tab);
     note_launch(2);
     return launch_status();
 }
