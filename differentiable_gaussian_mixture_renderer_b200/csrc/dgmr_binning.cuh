@@ -637,6 +637,12 @@ static __global__ void k_tile_ranges_from_counts(const uint32_t* __restrict__ ti
 // per round: after the ballots (which also ends the previous copy-out, so warp
 // 0 then advances the tile positions by the previous round's counts), after
 // the offsets, and after the staging.
+// The pairs are handed out by tile: a lane has its two tiles' ballots and walks
+// their set bits, so pairs of a tile come in rank order and need no rank of their
+// own.  By entry, each lane walking its entry's tiles, a warp waited for the
+// entry with the most tiles (up to 64) and looked every rank up: 65 us instead of 48
+// at 1M Gaussians, 1080p, 30 instead of 19 at 200k, 1024^2; with the tile ids left out
+// where nothing shows them (run_binning_grids), 557 -> 327 us for 12 batched views.
 constexpr unsigned kEmitStage = 4096;
 template <class Grids>
 static __global__ void __launch_bounds__(kChunkThreads) k_chunk_emit(const uint32_t* __restrict__ skey, const uint32_t* __restrict__ sval, uint32_t N,
@@ -653,8 +659,8 @@ static __global__ void __launch_bounds__(kChunkThreads) k_chunk_emit(const uint3
     __shared__ uint32_t roff[kSuperTiles + 1]; // start of each tile's run in the stage
     __shared__ uint32_t bal[kWarps][kSuperTiles];
     __shared__ uint32_t wpre[kWarps][kSuperTiles];
+    __shared__ uint32_t vals[kWarps][32]; // the round's entries
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t lt = (1u << lane) - 1u;
     uint32_t n_chunks = n_sort[2];
     n_chunks = n_chunks < rows.max_chunks ? n_chunks : rows.max_chunks;
     for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
@@ -677,6 +683,7 @@ static __global__ void __launch_bounds__(kChunkThreads) k_chunk_emit(const uint3
             const uint32_t b_hi = warp_bit_transpose(uint32_t(m >> 32), lane);
             bal[warp][lane] = b_lo;
             bal[warp][lane + 32] = b_hi;
+            vals[warp][lane] = g; // read by its own warp, before the copy-out's barrier
             __syncthreads(); // also ends the previous round's copy-out
             if (warp == 0) {
                 if (r0 != ch.a) { // the previous round's pairs advance each tile's position
@@ -712,22 +719,28 @@ static __global__ void __launch_bounds__(kChunkThreads) k_chunk_emit(const uint3
             __syncthreads();
             const uint32_t total = roff[kSuperTiles];
             const bool staged = total <= kEmitStage;
-            unsigned long long own = m;
-            while (own) {
-                const int k = __ffsll(static_cast<long long>(own)) - 1;
-                own &= own - 1ull;
-                const uint32_t rank = wpre[warp][k] + __popc(bal[warp][k] & lt);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t k = uint32_t(lane) + 32u * h;
+                uint32_t own = h == 0 ? b_lo : b_hi;
                 if (staged) {
-                    stage_val[roff[k] + rank] = g;
-                    stage_k[roff[k] + rank] = uint8_t(k);
-                } else {
+                    uint32_t at = roff[k] + wpre[warp][k];
+                    for (; own; own &= own - 1u, ++at) {
+                        stage_val[at] = vals[warp][__ffs(int(own)) - 1];
+                        stage_k[at] = uint8_t(k);
+                    }
+                } else if (own) {
                     const uint32_t t = tile_id[k];
-                    const uint32_t pos = base[k] + rank;
+                    uint32_t pos = base[k] + wpre[warp][k];
                     if (t == 0xffffffffu) {
                         flag_bounds(stats, 0x2bu);
-                    } else if (pos < cap) {
-                        out_tile[pos] = t;
-                        out_val[pos] = g;
+                    } else {
+                        for (; own; own &= own - 1u, ++pos)
+                            if (pos < cap) {
+                                if (out_tile)
+                                    out_tile[pos] = t;
+                                out_val[pos] = vals[warp][__ffs(int(own)) - 1];
+                            }
                     }
                 }
             }
@@ -739,7 +752,8 @@ static __global__ void __launch_bounds__(kChunkThreads) k_chunk_emit(const uint3
                 if (t == 0xffffffffu) {
                     flag_bounds(stats, 0x2bu);
                 } else if (pos < cap) {
-                    out_tile[pos] = t;
+                    if (out_tile)
+                        out_tile[pos] = t;
                     out_val[pos] = stage_val[i];
                 }
             }
@@ -826,12 +840,13 @@ static __global__ void __launch_bounds__(1024) k_tile_order(const int32_t* __res
 
 // Full binning: point_offsets (inclusive scan, reference order), depth sort,
 // super-tile entries and their sort, chunk counts, tile ranges and the point
-// list.  Returns the buffer index holding the point list (pair_val) and its
-// tile ids (pair_tile).  Requires b.perm = iota and b.depth_key filled by the
+// list.  Returns the buffer index holding the point list (pair_val) and, with
+// keep_tiles (the frame's views show them; no kernel reads them), its tile ids
+// (pair_tile).  Requires b.perm = iota and b.depth_key filled by the
 // preprocess.  n_super = super-tiles of all frames (super_count per frame).
 template <class T, class Grids>
 inline int run_binning_grids(uint32_t N, uint32_t n_tiles, uint32_t n_super, const Grids& grids, const uint32_t* tiles_touched, uint32_t* point_offsets,
-    const int32_t* rects, const T* xy, uint32_t cap, BinningBuffers& b, int32_t* ranges, uint32_t* stats, int n_sms, cudaStream_t stream, bool offsets_ready)
+    const int32_t* rects, const T* xy, uint32_t cap, BinningBuffers& b, int32_t* ranges, uint32_t* stats, int n_sms, cudaStream_t stream, bool offsets_ready, bool keep_tiles = false)
 {
     const ChainStream s(stream, N <= kChainMost);
     const int par = tile_sort_parity(n_super);
@@ -896,7 +911,7 @@ inline int run_binning_grids(uint32_t N, uint32_t n_tiles, uint32_t n_super, con
             smem_set = true;
         }
         launch_chained(k_chunk_emit<Grids>, cgrid, kChunkThreads, chunk_emit_smem(), s, b.pair_tile[spar], b.pair_val[spar], N, b.super_ranges, b.chunk_base, n_super,
-            b.n_sort, rows, b.tile_total, b.tile_incl, cap, b.pair_tile[1 - spar], b.pair_val[1 - spar], stats, grids);
+            b.n_sort, rows, b.tile_total, b.tile_incl, cap, keep_tiles ? b.pair_tile[1 - spar] : nullptr, b.pair_val[1 - spar], stats, grids);
         note_launch();
     } else {
         cudaMemsetAsync(ranges, 0, size_t(n_tiles) * 2 * sizeof(int32_t), s);
@@ -906,10 +921,10 @@ inline int run_binning_grids(uint32_t N, uint32_t n_tiles, uint32_t n_super, con
 
 template <class T>
 inline int run_binning(uint32_t N, unsigned gx, unsigned gy, const uint32_t* tiles_touched, uint32_t* point_offsets, const int32_t* rects, const T* xy,
-    uint32_t cap, BinningBuffers& b, int32_t* ranges, uint32_t* stats, int n_sms, cudaStream_t s, bool offsets_ready = false)
+    uint32_t cap, BinningBuffers& b, int32_t* ranges, uint32_t* stats, int n_sms, cudaStream_t s, bool offsets_ready = false, bool keep_tiles = false)
 {
     return run_binning_grids<T>(N, gx * gy, super_count(gx, gy), SingleGrid { gx, gy }, tiles_touched, point_offsets, rects, xy, cap, b, ranges, stats, n_sms, s,
-        offsets_ready);
+        offsets_ready, keep_tiles);
 }
 
 } // namespace dgmr

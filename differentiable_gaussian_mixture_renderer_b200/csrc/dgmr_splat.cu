@@ -1303,7 +1303,7 @@ void launch_render(const dgmr_scene* scene, const CameraT<float>& cam, float* fb
 {
     const uint32_t N = uint32_t(scene->n_gaussians);
     const int par
-        = run_binning<float>(N, cam.gx, cam.gy, L.tiles_touched, L.point_offsets, L.rects, L.xy, cap, L.bin, L.ranges, st_dev, num_sms(), s, true);
+        = run_binning<float>(N, cam.gx, cam.gy, L.tiles_touched, L.point_offsets, L.rects, L.xy, cap, L.bin, L.ranges, st_dev, num_sms(), s, true, true);
     launch_tile_order(L, par, N, cap, cam.gx * cam.gy, single_frame(cam, fb, L), s);
     launch_blend(kBlendSide, cam.gx * cam.gy, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, N, cap, st_dev, L.tile_order, single_frame(cam, fb, L), s);
 }
