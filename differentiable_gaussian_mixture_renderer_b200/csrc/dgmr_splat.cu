@@ -26,6 +26,7 @@ struct SplatLayout {
     float* xy;
     float* conic_opacity;
     uint32_t* tiles_touched;
+    uint2* tile_rect;
     uint32_t* point_offsets;
     int32_t* ranges;
     float* final_T;
@@ -53,6 +54,7 @@ inline SplatLayout splat_layout_n(uint32_t N, uint32_t n_tiles, size_t n_px, uin
     L.xy = c.take<float>(size_t(N) * 2);
     L.conic_opacity = c.take<float>(size_t(N) * 4);
     L.tiles_touched = c.take<uint32_t>(N);
+    L.tile_rect = c.take<uint2>(N);
     L.point_offsets = c.take<uint32_t>(N);
     L.ranges = c.take<int32_t>(size_t(n_tiles) * 2);
     L.final_T = c.take<float>(n_px);
@@ -92,6 +94,7 @@ struct SplatPre {
     float* xy;
     float* conic_opacity;
     uint32_t* tiles_touched;
+    uint2* tile_rect; // (x0 | y0 << 16, x1 | y1 << 16)
     uint32_t* depth_key;
     uint32_t* perm;
     float4* blend_rec;
@@ -100,14 +103,14 @@ struct SplatPre {
 
 // splat_forward.cu:70-118 for Gaussian i of the scene, written to output
 // slot o (o = i for one frame; o = the view's offset + i in a batch).
-// Bound by memory: 56 bytes in and 95 out per Gaussian at SH degree 0.  Every
+// Bound by memory: 56 bytes in and 103 out per Gaussian at SH degree 0.  Every
 // output is stored once, from the values of a Gaussian on no tile unless it
 // reaches one (stored first and overwritten: 40.7 us at 1M, now 37.6; 48
 // registers, 39.6 with 62 and 41 with 40).
 __device__ __forceinline__ void preprocess_one(const SplatPre& p, const CameraT<float>& cam, uint32_t i, uint32_t o)
 {
     int ex = 0, ey = 0;
-    unsigned touched = 0;
+    uint2 tile_rect = make_uint2(0u, 0u);
     float depth = 0.f;
     V2<float> xy = { 0.f, 0.f };
     V3<float> col = { 0.f, 0.f, 0.f };
@@ -123,8 +126,8 @@ __device__ __forceinline__ void preprocess_one(const SplatPre& p, const CameraT<
         ex = dgmr_fm::to_int_rz(dgmr_fm::ceil_f(3.f * dgmr_fm::sqrt_f(g.cov.v[0])));
         ey = dgmr_fm::to_int_rz(dgmr_fm::ceil_f(3.f * dgmr_fm::sqrt_f(g.cov.v[2])));
         const TileRect r = get_rect(g.centroid.x, g.centroid.y, ex, ey, cam.gx, cam.gy);
-        touched = (r.x1 - r.x0) * (r.y1 - r.y0);
-        if (touched != 0) {
+        if ((r.x1 - r.x0) * (r.y1 - r.y0) != 0) {
+            tile_rect = make_uint2(r.x0 | (r.y0 << 16), r.x1 | (r.y1 << 16));
             xy = g.centroid;
             const V3<float> campos = { cam.campos[0], cam.campos[1], cam.campos[2] };
             depth = len3(sub3(campos, mu));
@@ -141,7 +144,8 @@ __device__ __forceinline__ void preprocess_one(const SplatPre& p, const CameraT<
             r1 = make_float4(2.f * con.v[1], g.weight, q_cut, 0.f);
         }
     }
-    p.tiles_touched[o] = touched;
+    p.tiles_touched[o] = ((tile_rect.y & 0xffffu) - (tile_rect.x & 0xffffu)) * ((tile_rect.y >> 16) - (tile_rect.x >> 16));
+    p.tile_rect[o] = tile_rect;
     p.perm[o] = o;
     p.depth_key[o] = __float_as_uint(depth);
     reinterpret_cast<int2*>(p.rects)[o] = make_int2(ex, ey);
@@ -1103,7 +1107,7 @@ SplatPre make_pre(const dgmr_scene* scene, const SplatLayout& L)
 {
     return SplatPre { uint32_t(scene->n_gaussians), static_cast<const float*>(scene->centroids), static_cast<const float*>(scene->sh), scene->sh_stride,
         scene->sh_degree, static_cast<const float*>(scene->weights), static_cast<const float*>(scene->scales), static_cast<const float*>(scene->rotations),
-        L.rects, L.rgb, L.clamped, L.depths, L.xy, L.conic_opacity, L.tiles_touched, L.bin.depth_key, L.bin.perm, L.blend_rec,
+        L.rects, L.rgb, L.clamped, L.depths, L.xy, L.conic_opacity, L.tiles_touched, L.tile_rect, L.bin.depth_key, L.bin.perm, L.blend_rec,
         scene_formulation(scene, Formulation::Ots) };
 }
 
@@ -1303,7 +1307,7 @@ void launch_render(const dgmr_scene* scene, const CameraT<float>& cam, float* fb
 {
     const uint32_t N = uint32_t(scene->n_gaussians);
     const int par
-        = run_binning<float>(N, cam.gx, cam.gy, L.tiles_touched, L.point_offsets, L.rects, L.xy, cap, L.bin, L.ranges, st_dev, num_sms(), s, true, true);
+        = run_binning<float>(N, cam.gx, cam.gy, L.tiles_touched, L.point_offsets, L.rects, L.xy, cap, L.bin, L.ranges, st_dev, num_sms(), s, true, true, L.tile_rect);
     launch_tile_order(L, par, N, cap, cam.gx * cam.gy, single_frame(cam, fb, L), s);
     launch_blend(kBlendSide, cam.gx * cam.gy, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, N, cap, st_dev, L.tile_order, single_frame(cam, fb, L), s);
 }
@@ -1588,7 +1592,7 @@ dgmr_status make_batch(const dgmr_scene* scenes, int32_t n_scenes, const dgmr_ba
 
 SplatPre batch_pre(const SplatLayout& L, uint32_t G)
 {
-    return SplatPre { G, nullptr, nullptr, 1, 0, nullptr, nullptr, nullptr, L.rects, L.rgb, L.clamped, L.depths, L.xy, L.conic_opacity, L.tiles_touched,
+    return SplatPre { G, nullptr, nullptr, 1, 0, nullptr, nullptr, nullptr, L.rects, L.rgb, L.clamped, L.depths, L.xy, L.conic_opacity, L.tiles_touched, L.tile_rect,
         L.bin.depth_key, L.bin.perm, L.blend_rec, Formulation::Ots };
 }
 
@@ -1672,7 +1676,7 @@ dgmr_status dgmr_splat_batch_forward(const dgmr_scene* scenes, int32_t n_scenes,
     const uint32_t G = plan.tab.G, cap = uint32_t(pair_capacity);
     batch_preprocess(plan, st_dev, s);
     const int par = run_binning_grids<float>(G, plan.tab.n_tiles, plan.tab.n_stiles, plan.tab, L.tiles_touched, L.point_offsets, L.rects, L.xy, cap, L.bin, L.ranges, st_dev,
-        num_sms(), s, true);
+        num_sms(), s, true, false, L.tile_rect);
     launch_tile_order(L, par, G, cap, plan.tab.n_tiles, plan.tab, s);
     launch_blend(plan.blend_side, plan.tab.n_tiles, L.ranges, L.bin.pair_val[par], L.blend_rec, L.rgb, G, cap, st_dev, L.tile_order, plan.tab, s);
     note_launch();
