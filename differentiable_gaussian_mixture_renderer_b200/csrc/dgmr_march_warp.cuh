@@ -754,8 +754,10 @@ namespace dgmr {
 // Adjoint of one Gaussian's bin masses (grad/math.h:559-620), run by one lane
 // over the bins in shared memory -- in bin order, so its sums round exactly
 // as the one-thread loop does -- then added to the per-Gaussian accumulators.
+// Inlined at its one call: out of line it cost 5 % (31.0 ms instead of 29.1, forward +
+// backward at 100k, 512^2; 24.7 instead of 23.3 for 16 batched 64^2 views).
 template <class T>
-__device__ __noinline__ void lane_grad_entry(const VmMarch<T>& a, int32_t k, const Bin<T>* gbins, const T* borders, V3<T> o, V3<T> d, int live_end)
+__device__ __forceinline__ void lane_grad_entry(const VmMarch<T>& a, int32_t k, const Bin<T>* gbins, const T* borders, V3<T> o, V3<T> d, int live_end)
 {
     const RayEntry<T> en = load_entry(a, k);
     const V3<T> rgb = { a.rgb[3 * size_t(en.id)], a.rgb[3 * size_t(en.id) + 1], a.rgb[3 * size_t(en.id) + 2] };
