@@ -5,14 +5,17 @@
 // one thread per ray that work is a long dependent chain on one lane (with
 // the 127 bins in local memory), so the kernel ends up waiting on a few
 // rays while the SMs idle.  Here the 32 lanes of a warp share one ray:
-//  * the tile list is walked 32 entries at a time, one entry per lane
-//    (intersection with the ray, gates), results exchanged by shuffles;
+//  * the tile's list is cut down to the entries the ray can use, once (RayList);
+//    every pass walks those 32 at a time, one entry per lane (intersection with
+//    the ray, gates), results exchanged by shuffles;
 //  * lane l owns bins l, l+32, l+64, l+96 (four register bins); for each
 //    Gaussian, in list order, every lane evaluates the CDF at its own
 //    borders and takes the next border's value from its neighbour;
-//  * the strictly sequential parts -- section insertion (pass 1), sample
-//    positions, the blend and its adjoint peel -- run on every lane in
-//    lockstep from shared values, so no lane waits on another.
+//  * a section is inserted by the whole warp, lane i holding section i (pass 1),
+//    and the sample positions are written a section per lane;
+//  * the sequential parts -- the blend and its adjoint peel -- run on every
+//    lane in lockstep from shared values;
+//  * in the backward every lane runs one Gaussian's adjoint over its bins.
 // Per bin, Gaussian order and every arithmetic operation are those of the
 // one-thread loops (vol_marcher_forward.cu:295-501, math.h:412-468), so the
 // image is the same bits.  Warps are independent (no block barrier); blocks
@@ -483,9 +486,9 @@ __device__ __forceinline__ void warp_collect(SectionSet<kLargeSteps, T>& sec, Se
         return;
     }
     const uint32_t batches = ray_batches(rl, b, e);
+    const T from = sec.lo; // the same for the whole step
     for (uint32_t t = 0; t < batches; ++t) {
         const int32_t entry = ray_entry(rl, b, e, t, lane);
-        uint32_t m = __ballot_sync(0xffffffffu, entry >= 0);
         T depth = T(0), s0 = T(0), s1 = T(0), dt = T(0);
         bool ok = false;
         if (entry >= 0) {
@@ -494,34 +497,43 @@ __device__ __forceinline__ void warp_collect(SectionSet<kLargeSteps, T>& sec, Se
             const T sd = dgmr_fm::sqrt_f(g.C);
             depth = en.depth;
             const T mor = g.weight * en.mass;
-            ok = !(mor <= T(1.0f / 255.f) || mor > T(1000)) && !(g.C <= T(0)) && !dgmr_fm::isnan_f(g.centre);
             s0 = g.centre - sd * T(kRelevanceSigma);
             s1 = g.centre + sd * T(kRelevanceSigma);
             dt = ((sd * T(kRelevanceSigma)) * T(2)) / T(float(kStepsPerGaussian - 1));
+            ok = !(mor <= T(1.0f / 255.f) || mor > T(1000)) && !(g.C <= T(0)) && !dgmr_fm::isnan_f(g.centre);
+            // put() returns at once for a section outside [lo, hi): never walked
+            ok = ok && !(s1 <= from);
         }
-        const uint32_t okm = __ballot_sync(0xffffffffu, ok);
+        uint32_t m = __ballot_sync(0xffffffffu, ok);
+        // the walk ends before the first entry deeper than the set reaches at that
+        // point (`reach`, which only insertions change), so only entries to insert are
+        // walked: 1.684 -> 1.647 ms at 10k, 256^2, forward, 1.18 -> 1.155 ms in float64 at 4k,
+        // 97x65, with the backward; even with walking every entry at 100k, 512^2
+        T reach = sec.hi;
+        uint32_t deep = __ballot_sync(0xffffffffu, entry >= 0 && reach < depth);
         bool stop = false;
         while (m) {
             const int j = __ffs(int(m)) - 1;
             m &= m - 1u;
-            const T dj = __shfl_sync(0xffffffffu, depth, j);
-            if (sec.hi < dj) {
+            if (deep & lanes_below(j + 1)) {
                 stop = true;
                 break;
             }
-            if (!((okm >> j) & 1u))
-                continue;
             const Section<T> sj = { __shfl_sync(0xffffffffu, s0, j), __shfl_sync(0xffffffffu, s1, j), __shfl_sync(0xffffffffu, dt, j) };
-            // put() returns at once for a section outside [lo, hi) and leaves the
-            // set unchanged for a covered one: skip both without the call
-            if (sj.end <= sec.lo || sj.start >= sec.hi || warp_section_covered(sec, sj, lane))
+            // (hi may have come in; put() leaves the set unchanged for a covered section)
+            if (sj.start >= sec.hi || warp_section_covered(sec, sj, lane))
                 continue;
             if (kPut == PutMode::Inline)
                 warp_put(sec, pieces, sj, lane);
             else
                 warp_put_call(sec, pieces, sj, lane);
+            const T hi = sec.hi;
+            if (hi < reach) {
+                deep = __ballot_sync(0xffffffffu, entry >= 0 && hi < depth) & ~lanes_below(j + 1);
+                reach = hi;
+            }
         }
-        if (stop)
+        if (stop || deep)
             break;
     }
 }
