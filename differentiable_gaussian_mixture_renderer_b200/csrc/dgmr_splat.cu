@@ -54,12 +54,13 @@ inline SplatLayout splat_layout_n(uint32_t N, uint32_t n_tiles, size_t n_px, uin
     L.xy = c.take<float>(size_t(N) * 2);
     L.conic_opacity = c.take<float>(size_t(N) * 4);
     L.tiles_touched = c.take<uint32_t>(N);
-    L.tile_rect = c.take<uint2>(N);
     L.point_offsets = c.take<uint32_t>(N);
     L.ranges = c.take<int32_t>(size_t(n_tiles) * 2);
     L.final_T = c.take<float>(n_px);
     L.n_contrib = c.take<int32_t>(n_px);
     L.grad_acc = c.take<double>(size_t(N) * 9);
+    // from the preprocess to the binning only; the backward, which follows both, zeroes grad_acc first
+    L.tile_rect = reinterpret_cast<uint2*>(L.grad_acc);
     L.blend_rec = c.take<float4>(size_t(N) * 2);
     L.tile_order = c.take<uint32_t>(n_tiles);
     L.tile_cost = c.take<uint32_t>(n_tiles);
