@@ -44,7 +44,7 @@ struct VmLayout {
     uint32_t* stats;
     uint32_t* pre_scan_tmp;
     double* acc; // backward, [N,13]: mass, rgb(3), inverse covariance(6), centroid(3)
-    float4* rec; // float only, [N,5]: the march's records (k_vm_records)
+    float4* rec; // float, [N,5]: the march's records (k_vm_records)
     BinningBuffers bin;
     size_t pre_bytes;
     size_t bytes;
@@ -65,7 +65,7 @@ inline VmLayout<T> vm_layout(uint32_t N, uint32_t n_tiles, uint32_t cap, void* b
     L.pre_scan_tmp = c.take<uint32_t>(scan_temp_bytes(N) / 4 + 8); // + room for k_pair_count's eight counters
     L.pre_bytes = c.off;
     L.acc = c.take<double>(size_t(N) * kVmAcc);
-    L.rec = c.take<float4>(sizeof(T) == 4 ? size_t(N) * kMarchRec : 0);
+    L.rec = c.take<float4>(size_t(N) * kMarchRec); // in double unused: a workspace of either type's size serves both
     carve_binning(c, L.bin, N, n_tiles, cap);
     L.bytes = c.off;
     return L;
