@@ -482,7 +482,7 @@ def run_ours(args):
                     "h2d_bytes_per_step": args.batch * 8 * (16 + 16 + 3 + 3 + 3 + 1),
                     "d2h_bytes_per_step": args.batch * 3 * args.width * args.height * 4,
                     "p50_ms": pct(lat_e2e, 50), "p99_ms": pct(lat_e2e, 99)},
-            "roofline": {"kernel": "k_splat_blend", "bound": "hbm", "achieved": achieved, "peak": peak,
+            "roofline": {"kernel": "k_splat_blend_quarters", "bound": "hbm", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
                          "ms_per_launch": blend_ms, "n_pairs": n_pairs, "algorithmic_bytes": blend_bytes,
                          "bytes_formula": "40 P + 8 T + 12 px",

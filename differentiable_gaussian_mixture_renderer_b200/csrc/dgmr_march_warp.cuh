@@ -31,7 +31,7 @@ constexpr unsigned kRayRounds = 4; // 4 x 32 lanes = 128 borders
 template <class T>
 constexpr unsigned kRayList = sizeof(T) == 4 ? 1024 : 512; // list entries a ray can use that its warp keeps (RayList; 48 KB per block)
 
-// A ray's section set lives in shared memory, once per warp: lane 0 inserts,
+// A ray's section set lives in shared memory, once per warp: the warp inserts,
 // every lane reads it after a __syncwarp (kept per lane, the 32 identical
 // copies and the insertion's scratch went to local memory).
 template <class T>
