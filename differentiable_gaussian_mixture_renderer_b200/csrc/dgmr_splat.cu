@@ -711,6 +711,18 @@ struct BwdPixels {
     int32_t n0, n1; // contributors
 };
 
+// Whether the packed walk's products with an unused record are exact zeros for
+// what the lane's pixels have collected so far.
+__device__ __forceinline__ bool plain_state(const BwdPixels& p)
+{
+    const auto both = [](F2 t) {
+        float lo, hi;
+        split2(t, &lo, &hi);
+        return plain_value(lo) && plain_value(hi);
+    };
+    return both(p.Tr) && both(p.a0) && both(p.a1) && both(p.a2);
+}
+
 // One record on the lane's two pixels: `use` says which of them it reaches.
 // Returns whether any partial is nonzero.  kGuarded: values may be huge or not
 // finite, and a pixel that does not use the record must not see them.
@@ -934,6 +946,10 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 5) k_splat_bwd_pixels(const in
             for (int k = 0; k < 12; ++k)
                 held[k] = v[k];
         }
+        // a record of the guarded walk may leave a state that is not plain, which
+        // the records in front meet: the rest of the walk is then guarded too
+        if (guarded && plain)
+            plain = __all_sync(0xffffffffu, plain_state(p));
     }
     add(warp_reduce_scatter12(held, lane));
 }

@@ -1,0 +1,60 @@
+"""What a splat with a non-finite or very large colour leaves behind in the
+backward's walk -- the colour behind the next record, on the pixels that it covers
+-- stays with those pixels: the gradients of Gaussians that share no pixel with
+it are those of the scene with an ordinary colour there."""
+import numpy as np
+import pytest
+import torch
+
+from differentiable_gaussian_mixture_renderer_b200 import scene as S, splat
+from test_gpu_parity import GRAD_TOL, grad_err, run_splat
+
+pytestmark = pytest.mark.gpu
+
+GRAD_NAMES = ("sh", "weights", "centroids", "scales", "rotations")
+W, H = 64, 48
+
+
+def reach_of(v):
+    """[N, H, W]: alpha reaches 1/255 there, with a margin on the cutoff."""
+    xy, co = v["points_xy_image"].astype(np.float64), v["conic_opacity"].astype(np.float64)
+    dx = np.arange(W)[None, None, :] - xy[:, 0, None, None]
+    dy = np.arange(H)[None, :, None] - xy[:, 1, None, None]
+    q = co[:, 0, None, None] * dx ** 2 + 2 * co[:, 1, None, None] * dx * dy + co[:, 2, None, None] * dy ** 2
+    return (v["tiles_touched"] > 0)[:, None, None] & (co[:, 3, None, None] * np.exp(-0.5 * q) > 0.99 / 255)
+
+
+def deep_splat(v, reach):
+    """The Gaussian on the fewest pixels of those that contribute to one, with at
+    least 64 entries before it in that tile's list."""
+    best = None
+    for g in np.flatnonzero(reach.any((1, 2))):
+        for y, x in zip(*np.nonzero(reach[g])):
+            b, e = v["i_ranges"][(y // 16) * (W // 16) + x // 16]
+            at = np.flatnonzero(v["point_list"][b:e] == g)  # empty past the rectangle's tiles
+            if at.size and 64 <= at[0] < v["n_contrib"][y, x]:
+                n = int(reach[g].sum())
+                best = (n, g) if best is None or n < best[0] else best
+                break
+    return best[1]
+
+
+@pytest.mark.parametrize("value,scale", [(float("inf"), 1.0), (float("nan"), 1.0), (3e38, 1e6)])
+def test_a_huge_colour_stays_with_its_pixels(cuda, value, scale):
+    sc = S.make_scene(1500, seed=3)
+    cam = S.make_camera(W, H)
+    G = torch.tensor(np.random.default_rng(1).normal(size=(3, H, W)) * scale, dtype=torch.float32, device=cuda)
+    _, frame, ts = run_splat(sc, cam, cuda)
+    v = {k: t.cpu().numpy() for k, t in frame.views().items()}
+    reach = reach_of(v)
+    bad = deep_splat(v, reach)
+    apart = ~(reach & reach[bad]).any((1, 2))
+    assert 0 < reach[bad].sum() < 64 and apart.sum() > 1000
+    clean = splat.splat_backward(frame, G, *ts)
+    sc.sh[bad, 0, 0] = value
+    _, frame, ts = run_splat(sc, cam, cuda)
+    dirty = splat.splat_backward(frame, G, *ts)
+    for name, a, b in zip(GRAD_NAMES, clean, dirty):
+        a, b = (t.cpu().numpy().reshape(sc.n, -1)[apart] for t in (a, b))
+        assert np.isfinite(b).all(), (name, int((~np.isfinite(b)).any(1).sum()))
+        assert grad_err(b, a) <= GRAD_TOL, name
