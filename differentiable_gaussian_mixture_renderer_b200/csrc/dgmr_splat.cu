@@ -240,14 +240,17 @@ __device__ __forceinline__ float rect_min_q(float cx, float cy, float a, float b
 
 // The packed walks (two pixels per lane, the halves of packed floats) take
 // records and pixels of ordinary magnitude: the half that does not use a record is
-// multiplied by an exact zero, which needs finite operands (products of two
-// values up to kPlain are finite), and its exp is evaluated without the tests for
-// special cases.  So the conic has to be positive definite, and close enough to
-// the 8x8 quarter for the rounding of the quadratic form (4 ulp of its terms) to
-// stay far above the -170 where exp(-q/2) overflows, and q_cut (NaN for a negative
-// opacity) to keep it off the range where the exp is subnormal; it bounds the
-// opacity too, by e^50 / 255.  Other records take the guarded walk.
-constexpr float kPlain = 1.0e18f, kPlainForm = 1.0e8f, kPlainCut = 100.f;
+// multiplied by an exact zero, which needs finite operands, and its exp is
+// evaluated without the tests for special cases.  The largest operand is the
+// backward's product of four: transmittance (kPlainT), the distance of a colour
+// from the one behind (3 x 2 kPlain over the channels), the image gradient
+// (kPlain) and the opacity (at most e^50 / 255 = 2.1e19 by kPlainCut), together
+// below 3e36.  The conic has to be positive definite, and close enough to the
+// 8x8 quarter for the rounding of the quadratic form (4 ulp of its terms) to stay
+// far above the -170 where exp(-q/2) overflows, and q_cut (NaN for a negative
+// opacity) to keep it off the range where the exp is subnormal.  Other records take
+// the guarded walk.
+constexpr float kPlain = 1.0e8f, kPlainT = 2.f, kPlainForm = 1.0e8f, kPlainCut = 100.f;
 __device__ __forceinline__ bool plain_value(float x) { return fabsf(x) <= kPlain; } // false for NaN
 __device__ __forceinline__ bool plain_record(float4 r0, float4 r1, float4 rgb, float x0, float y0)
 {
@@ -715,12 +718,12 @@ struct BwdPixels {
 // what the lane's pixels have collected so far.
 __device__ __forceinline__ bool plain_state(const BwdPixels& p)
 {
-    const auto both = [](F2 t) {
+    const auto both = [](F2 t, float most) {
         float lo, hi;
         split2(t, &lo, &hi);
-        return plain_value(lo) && plain_value(hi);
+        return fabsf(lo) <= most && fabsf(hi) <= most; // false for NaN
     };
-    return both(p.Tr) && both(p.a0) && both(p.a1) && both(p.a2);
+    return both(p.Tr, kPlainT) && both(p.a0, kPlain) && both(p.a1, kPlain) && both(p.a2, kPlain);
 }
 
 // One record on the lane's two pixels: `use` says which of them it reaches.
@@ -862,7 +865,7 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 5) k_splat_bwd_pixels(const in
     p.bg = f2(bg[0], bg[1]);
     p.n0 = n[0];
     p.n1 = n[1];
-    plain = __all_sync(0xffffffffu, plain);
+    plain = __all_sync(0xffffffffu, plain && plain_state(p));
     const int32_t b = ranges[2 * tile];
     const int32_t end = __reduce_max_sync(0xffffffffu, max(n[0], n[1]));
     const float fpx = float(px);

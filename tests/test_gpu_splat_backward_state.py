@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from differentiable_gaussian_mixture_renderer_b200 import scene as S, splat
-from test_gpu_parity import GRAD_TOL, grad_err, run_splat
+from test_gpu_parity import GRAD_TOL, cam_tensors, grad_err, run_splat, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -57,4 +57,38 @@ def test_a_huge_colour_stays_with_its_pixels(cuda, value, scale):
     for name, a, b in zip(GRAD_NAMES, clean, dirty):
         a, b = (t.cpu().numpy().reshape(sc.n, -1)[apart] for t in (a, b))
         assert np.isfinite(b).all(), (name, int((~np.isfinite(b)).any(1).sum()))
+        assert grad_err(b, a) <= GRAD_TOL, name
+
+
+def test_a_huge_product_stays_with_its_pixel(cuda):
+    """A splat with an opacity of 1e12 and a colour of 1e15 next to a pixel that it
+    does not reach, whose image gradient is 8e17: each is finite, their product is
+    not, and none of it belongs to the splat."""
+    sc = S.make_scene(1500, seed=3)
+    cam = S.make_camera(W, H)
+    shs, w, mu, s, q = to_dev(sc, cuda)
+    view, proj, campos, bg = cam_tensors(cam, cuda)
+
+    def run():
+        _, frame = splat.splat_forward(shs, w, mu, s, q, view, proj, campos, bg, W, H, cam.tan_fovx, cam.tan_fovy, 0, formulation="opacity")
+        return frame, {k: t.cpu().numpy() for k, t in frame.views().items()}
+
+    _, v = run()
+    # nearest to the middle of an 8x8 quarter, and inside the frame
+    xy = v["points_xy_image"]
+    mid = np.abs(xy % 8 - 3.5).max(1) + 1e3 * ((v["tiles_touched"] == 0) | (xy < 0).any(1) | (xy > (W - 1, H - 1)).any(1))
+    g = int(mid.argmin())
+    w[g], shs[g, 0, :], s[g] = 1e12, 1e15, 1e-4
+    frame, v = run()
+    reach = reach_of(v)[g]
+    x0, y0 = (int(c) // 8 * 8 for c in xy[g])
+    quarter = reach[y0:y0 + 8, x0:x0 + 8]
+    assert quarter.any() and not quarter[0, 0]
+    G = torch.tensor(np.random.default_rng(1).normal(size=(3, H, W)), dtype=torch.float32, device=cuda)
+    want = splat.splat_backward(frame, G, shs, w, mu, s, q)
+    G[:, y0, x0] = 8e17
+    got = splat.splat_backward(frame, G, shs, w, mu, s, q)
+    for name, a, b in zip(GRAD_NAMES, want, got):
+        a, b = a[g].cpu().numpy(), b[g].cpu().numpy()
+        assert np.isfinite(a).all() and np.isfinite(b).all(), (name, a, b)
         assert grad_err(b, a) <= GRAD_TOL, name
