@@ -778,28 +778,30 @@ __device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, f
     const F2 na0 = add2(mul2_rounded(alpha, f2(c.x)), mul2_rounded(keep, p.a0));
     const F2 na1 = add2(mul2_rounded(alpha, f2(c.y)), mul2_rounded(keep, p.a1));
     const F2 na2 = add2(mul2_rounded(alpha, f2(c.z)), mul2_rounded(keep, p.a2));
-    const auto halves = [&](F2 t, float* lo, float* hi) {
+    // a saturated pixel has no gradient but the colour's, whatever the opacity (it may be infinite) or the exponent
+    const bool live0 = use0 && og0 < 0.99f, live1 = use1 && og1 < 0.99f;
+    const auto halves = [&](F2 t, bool take0, bool take1, float* lo, float* hi) {
         split2(t, lo, hi);
         if (kGuarded) {
-            *lo = use0 ? *lo : 0.f;
-            *hi = use1 ? *hi : 0.f;
+            *lo = take0 ? *lo : 0.f;
+            *hi = take1 ? *hi : 0.f;
         }
     };
-    const auto sum = [&](F2 t) {
+    const auto sum = [&](F2 t, bool take0, bool take1) {
         float lo, hi;
-        halves(t, &lo, &hi);
+        halves(t, take0, take1, &lo, &hi);
         return lo + hi;
     };
     // in the order of k_splat_bwd_pixels' accumulators
-    v[0] = sum(gx);
-    v[1] = sum(gy);
-    halves(gxx, &v[2], &v[3]);
-    halves(gxy, &v[4], &v[5]);
-    halves(gyy, &v[6], &v[7]);
-    v[8] = sum(go);
-    v[9] = sum(w0);
-    v[10] = sum(w1);
-    v[11] = sum(w2);
+    v[0] = sum(gx, live0, live1);
+    v[1] = sum(gy, live0, live1);
+    halves(gxx, live0, live1, &v[2], &v[3]);
+    halves(gxy, live0, live1, &v[4], &v[5]);
+    halves(gyy, live0, live1, &v[6], &v[7]);
+    v[8] = sum(go, live0, live1);
+    v[9] = sum(w0, use0, use1);
+    v[10] = sum(w1, use0, use1);
+    v[11] = sum(w2, use0, use1);
     if (kGuarded) {
         const auto pick = [&](F2& to, F2 from) {
             float a, b, x, y;

@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from differentiable_gaussian_mixture_renderer_b200 import scene as S, splat
+from oracle import oracle as O
 from test_gpu_parity import GRAD_TOL, cam_tensors, grad_err, run_splat, to_dev
 
 pytestmark = pytest.mark.gpu
@@ -92,3 +93,22 @@ def test_a_huge_product_stays_with_its_pixel(cuda):
         a, b = a[g].cpu().numpy(), b[g].cpu().numpy()
         assert np.isfinite(a).all() and np.isfinite(b).all(), (name, a, b)
         assert grad_err(b, a) <= GRAD_TOL, name
+
+
+@pytest.mark.parametrize("weight", [3e38, float("inf"), float("nan")])
+def test_a_saturated_splat_has_the_oracles_gradients(cuda, weight):
+    """An opacity that overflows (3e38 does, in the Ots formulation) leaves its splat
+    saturated on every pixel: its opacity, centre and shape have no gradient."""
+    sc = S.make_scene(1500, seed=3)
+    sc.weights[100] = weight
+    cam = S.make_camera(W, H)
+    G = np.random.default_rng(1).normal(size=(3, H, W)).astype(np.float32)
+    ref = O.splat_forward(sc, cam)
+    assert not np.isfinite(ref["conic_opacity"][100, 3]) and ref["tiles_touched"][100] > 0
+    gref = O.splat_backward(sc, cam, ref, G)
+    _, frame, ts = run_splat(sc, cam, cuda)
+    for name, g in zip(GRAD_NAMES, splat.splat_backward(frame, torch.tensor(G, device=cuda), *ts)):
+        g, want = g.cpu().numpy().reshape(gref[name].shape), gref[name]
+        fine = np.isfinite(want)
+        assert np.isfinite(g[fine]).all(), name
+        assert grad_err(g[fine], want[fine]) <= GRAD_TOL, name
