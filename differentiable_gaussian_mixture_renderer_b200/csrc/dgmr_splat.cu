@@ -656,8 +656,8 @@ void launch_blend(int side, uint32_t n_tiles, const int32_t* ranges, const uint3
 // holds at every butterfly level (12 -> 6 -> 3, the upper half kept by the lanes
 // whose level bit is set), exchange one pair of the three and sum the third,
 // then halve the two that are left.  Every sum is the tree over lane distances 16,
-// 8, 4, 2, 1.  Lane l returns the warp total of slot reduce_slot(l), lanes
-// that differ in bit 0 the same one.
+// 8, 4, 2.  Lane l returns slot reduce_slot(l)'s sum over the 16 lanes of its own
+// parity.
 __device__ __forceinline__ int reduce_slot(int lane)
 {
     const int base = 6 * ((lane >> 4) & 1) + 3 * ((lane >> 3) & 1);
@@ -676,8 +676,7 @@ __device__ __forceinline__ float warp_reduce_scatter12(const float (&v)[12], int
     // slots 0 and 1 of the three between the lanes of bit 2; slot 2 on both
     const float c = (b2 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, b2 ? b[0] : b[1], 4);
     const float d = b[2] + __shfl_xor_sync(0xffffffffu, b[2], 4);
-    const float e = (b1 ? d : c) + __shfl_xor_sync(0xffffffffu, b1 ? c : d, 2);
-    return e + __shfl_xor_sync(0xffffffffu, e, 1);
+    return (b1 ? d : c) + __shfl_xor_sync(0xffffffffu, b1 ? c : d, 2);
 }
 
 // Reverse-order blend adjoint.  A warp owns an 8x8 quarter of a tile and a lane
@@ -689,9 +688,14 @@ __device__ __forceinline__ float warp_reduce_scatter12(const float (&v)[12], int
 // moments of g_q = d/dq over its pixels (g_q dx and g_q dy, from which
 // k_splat_bwd_gaussians takes the centre's gradient), the conic's gradients (g_q
 // dx^2, 2 g_q dx dy, g_q dy^2), d/dopacity and d/drgb, and twelve lanes add one
-// value each.  The conic's three are summed over 32 pixels at a time, upper and
-// lower half apart: the chain to a long thin splat's scales cancels by 10^5, and
-// with a float sum over 64 pixels single elements moved by 1e-3.  The totals over warps are double: in float,
+// value each.  A float sum covers 32 pixels, the even or the odd columns of the
+// quarter, which meet in double; the conic's three cover 16, upper and lower half
+// apart: the chain to a long thin splat's scales cancels by 10^5, and with float
+// sums over 64 pixels single elements moved by 1e-3.  (Distance from per-pixel
+// double sums, mean of 32 frames in the 2-norm: colours 5.8e-8, opacities 6.3e-8;
+// 6.5e-8 and 7.0e-8 with float sums over 64 pixels, 6.0e-8 and 6.5e-8 over 32 as 8x4
+// blocks; the same time as over 64, a
+// tenth less than per 8x4 block.)  The totals over warps are double too: in float,
 // the order in which the atomics of many cancelling terms land moved single
 // elements by ~1e-3 relative from run to run at 200k Gaussians, 1024^2.
 // Tiles run in the forward's launch order (heaviest predicted walk first); a
@@ -879,9 +883,10 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 5) k_splat_bwd_pixels(const in
     const int slot = reduce_slot(lane);
     const int my_slot = slot < 2 ? slot : slot < 8 ? 1 + slot / 2 : slot - 3;
     const bool adds = (lane & 1) == 0 && ((lane & 2) == 0 || (lane & 4) == 0); // slot 2 of three is on both lanes of bit 2
-    const auto add = [&](float total) {
-        if (adds && held_id != 0xffffffffu && total != 0.f)
-            atomicAdd(acc + size_t(held_id) * 9 + my_slot, double(total));
+    const auto add = [&](float part) {
+        const double total = double(part) + double(__shfl_xor_sync(0xffffffffu, part, 1));
+        if (adds && held_id != 0xffffffffu && total != 0.0)
+            atomicAdd(acc + size_t(held_id) * 9 + my_slot, total);
     };
     ListWalk next;
     next.id = ListWalk::entry(list + b, end - 32 + lane, 0, end);
