@@ -31,7 +31,7 @@ struct SplatLayout {
     int32_t* ranges;
     float* final_T;
     int32_t* n_contrib;
-    double* grad_acc; // [N,9]: d/dq times (dx, dy, dx^2, 2 dx dy, dy^2), opacity, rgb(3), summed over pixels in double
+    double* grad_acc; // [N,9]: xy(2) conic(3) opacity rgb(3), summed over pixels in double
     float4* blend_rec; // [N,2]: (x, y, a, c), (2b, opacity, q_cut, 0) -- the blend's 32-byte record
     uint32_t* tile_order; // [tiles] launch order of the per-tile kernels, heaviest first
     uint32_t* tile_cost; // [tiles] predicted blend cost of each tile as a bucket, 0 = heaviest
@@ -685,19 +685,20 @@ __device__ __forceinline__ float warp_reduce_scatter12(const float (&v)[12], int
 // packed operation for both, and a record's partials are summed over 64 pixels
 // by one warp reduction.  Each pixel walks its contributors back to front,
 // recovering T_i = T_{i+1} / (1 - alpha_i).  Per record the warp sums the
-// moments of g_q = d/dq over its pixels (g_q dx and g_q dy, from which
-// k_splat_bwd_gaussians takes the centre's gradient), the conic's gradients (g_q
-// dx^2, 2 g_q dx dy, g_q dy^2), d/dopacity and d/drgb, and twelve lanes add one
-// value each.  A float sum covers 32 pixels, the even or the odd columns of the
-// quarter, which meet in double; the conic's three cover 16, upper and lower half
-// apart: the chain to a long thin splat's scales cancels by 10^5, and with float
-// sums over 64 pixels single elements moved by 1e-3.  (Distance from per-pixel
-// double sums, mean of 32 frames in the 2-norm: colours 5.8e-8, opacities 6.3e-8;
-// 6.5e-8 and 7.0e-8 with float sums over 64 pixels, 6.0e-8 and 6.5e-8 over 32 as 8x4
-// blocks; the same time as over 64, a
-// tenth less than per 8x4 block.)  The totals over warps are double too: in float,
-// the order in which the atomics of many cancelling terms land moved single
-// elements by ~1e-3 relative from run to run at 200k Gaussians, 1024^2.
+// gradients of the centre, the conic, the opacity and the colour over its pixels,
+// and twelve lanes add one value each.  A float sum covers 32 pixels, the even or
+// the odd columns of the quarter, which meet in double; the conic's three cover
+// 16, upper and lower half apart: the chain to a long thin splat's scales cancels
+// by 10^5, and with float sums over 64 pixels single elements moved by 1e-3.  The
+// totals over warps are double too: in float, the order in which the atomics of
+// many cancelling terms land moved single elements by ~1e-3 relative from run to
+// run at 200k Gaussians, 1024^2.
+// Distance from per-pixel double sums, mean of 32 frames in the 2-norm: colours
+// 5.8e-8, opacities 6.3e-8, centres 8.4e-8; with float sums over 64 pixels 6.5e-8
+// and 7.0e-8, in the time of the columns; over 32 pixels as 8x4 blocks 6.0e-8 and
+// 6.5e-8, in a tenth more.  The centre's gradient from the moments g_q dx and g_q
+// dy, multiplied by the conic once per Gaussian, is 1.3e-7 off (the products
+// cancel after the sums are rounded), in 2.5 % less time.
 // Tiles run in the forward's launch order (heaviest predicted walk first); a
 // warp walks its tile's list only up to its own pixels' last contributor.
 //
@@ -706,7 +707,7 @@ __device__ __forceinline__ float warp_reduce_scatter12(const float (&v)[12], int
 // 80 registers without spills beat 64 with them, and the next batch is requested
 // ahead (ListWalk: 299 -> 273 us at 1M, 1080p, 284 -> 288 at 200k, 1024^2).  Against a
 // pixel per lane, a reduction per 32 pixels of all nine values and 48 registers:
-// 406 -> 273 us at 1M, 1080p; 430 -> 288 us at 200k, 1024^2.
+// 401 -> 281 us at 1M, 1080p; 430 -> 299 us at 200k, 1024^2.
 constexpr int kBwdWarps = 4; // the quarters of a tile
 static_assert(kTile == 16, "four 8x8 quarters per tile");
 
@@ -716,6 +717,13 @@ struct BwdPixels {
     F2 g0, g1, g2; // image gradient
     F2 bg; // final T times the gradient's product with the background
     int32_t n0, n1; // contributors
+};
+
+// A record's quadratic form on the lane's two pixels, q = x dx + y dy, in splat_q's operations.
+struct BwdForm {
+    F2 x; // a dx + 2b dy
+    F2 y; // c dy
+    F2 q;
 };
 
 // Whether the packed walk's products with an unused record are exact zeros for
@@ -734,14 +742,14 @@ __device__ __forceinline__ bool plain_state(const BwdPixels& p)
 // Returns whether any partial is nonzero.  kGuarded: values may be huge or not
 // finite, and a pixel that does not use the record must not see them.
 template <bool kGuarded>
-__device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, float4 c, F2 q, float dx, F2 dy, bool use0, bool use1, float (&v)[12])
+__device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, float4 c, const BwdForm& f, float dx, F2 dy, bool use0, bool use1, float (&v)[12])
 {
     const float op = r1.y;
     float e0, e1;
-    split2(exp2_nonpos(mul2(q, f2(-0.5f))), &e0, &e1);
+    split2(exp2_nonpos(mul2(f.q, f2(-0.5f))), &e0, &e1);
     if (kGuarded) {
         float q0, q1;
-        split2(q, &q0, &q1);
+        split2(f.q, &q0, &q1);
         if (use0 && !(q0 >= -170.f && q0 <= 170.f))
             e0 = dgmr_fm::exp_f_nonpos(-0.5f * q0);
         if (use1 && !(q1 >= -170.f && q1 <= 170.f))
@@ -777,6 +785,8 @@ __device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, f
     const F2 go = mul2(f2(ga0, ga1), g); // d/dopacity
     const F2 gq = mul2(mul2(g, f2(-0.5f)), mul2(f2(ga0, ga1), f2(op)));
     const F2 gx = mul2(gq, f2(dx)), gy = mul2(gq, dy);
+    // d/dcentre = -g_q (2a dx + 2b dy, 2c dy + 2b dx)
+    const F2 ux = fma2(f2(-r0.z), f2(dx), mul2(f.x, neg)), uy = fma2(f.y, f2(-2.f), f2(-r1.x * dx));
     const F2 gxx = mul2(gx, f2(dx)), gxy = mul2(mul2(gx, f2(2.f)), dy), gyy = mul2(gy, dy);
     const F2 keep = f2(x0, x1); // 1 - alpha
     const F2 na0 = add2(mul2_rounded(alpha, f2(c.x)), mul2_rounded(keep, p.a0));
@@ -797,8 +807,8 @@ __device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, f
         return lo + hi;
     };
     // in the order of k_splat_bwd_pixels' accumulators
-    v[0] = sum(gx, live0, live1);
-    v[1] = sum(gy, live0, live1);
+    v[0] = sum(mul2(gq, ux), live0, live1);
+    v[1] = sum(mul2(gq, uy), live0, live1);
     halves(gxx, live0, live1, &v[2], &v[3]);
     halves(gxy, live0, live1, &v[4], &v[5]);
     halves(gyy, live0, live1, &v[6], &v[7]);
@@ -929,9 +939,12 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 5) k_splat_bwd_pixels(const in
             // splat_q on both pixels
             const float dx = fpx - q0.x;
             const F2 dy = add2(fpy, f2(-q0.y));
-            const F2 q = fma2(fma2(f2(q0.z), f2(dx), mul2(f2(q1.x), dy)), f2(dx), mul2(mul2(f2(q0.w), dy), dy));
+            BwdForm form;
+            form.x = fma2(f2(q0.z), f2(dx), mul2(f2(q1.x), dy));
+            form.y = mul2(f2(q0.w), dy);
+            form.q = fma2(form.x, f2(dx), mul2(form.y, dy));
             float qa, qb;
-            split2(q, &qa, &qb);
+            split2(form.q, &qa, &qb);
             // the forward's cutoff: past q_cut alpha < 1/255, so exp is not
             // needed; a record no lane of the warp needs costs one vote
             const bool u0 = kk < p.n0 && !(qa > q1.z), u1 = kk < p.n1 && !(qb > q1.z);
@@ -943,10 +956,10 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 5) k_splat_bwd_pixels(const in
             float v[12], w;
             bool any;
             if (guarded) {
-                any = bwd_record<true>(p, q0, q1, col, q, dx, dy, u0, u1, v);
+                any = bwd_record<true>(p, q0, q1, col, form, dx, dy, u0, u1, v);
                 w = warp_reduce_scatter12(held, lane);
             } else {
-                any = bwd_record<false>(p, q0, q1, col, q, dx, dy, u0, u1, v);
+                any = bwd_record<false>(p, q0, q1, col, form, dx, dy, u0, u1, v);
                 w = warp_reduce_scatter12(held, lane);
             }
             add(w);
@@ -1052,20 +1065,16 @@ __device__ __forceinline__ void store_sh_rows(const SplatBwdGauss& p, const floa
 template <bool kAddSh>
 __device__ __forceinline__ void bwd_gaussian_one(const SplatBwdGauss& p, const CameraT<float>& cam, uint32_t i, uint32_t o, GaussianGrads& sum, float* row)
 {
-    double m[9];
+    float a[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k)
-        m[k] = p.acc[size_t(o) * 9 + k];
+        a[k] = float(p.acc[size_t(o) * 9 + k]);
     const V3<float> mu = { p.centroids[3 * i], p.centroids[3 * i + 1], p.centroids[3 * i + 2] };
     const V3<float> sc = mul3(V3<float> { p.scales[3 * i], p.scales[3 * i + 1], p.scales[3 * i + 2] }, cam.cov_scale_multiplier);
     const float* q = p.rotations + 4 * size_t(i);
     const M3<float> R = quat_to_mat3(q[0], q[1], q[2], q[3]);
     const Gaussian2d<float> g2 = splat_project(p.form, p.weights[i], mu, sc, R, cam, 0.3f);
     const S2<float> M = inverse2(g2.cov);
-    // q = a dx^2 + 2b dx dy + c dy^2 with d = pixel - centre: the centre's
-    // gradient from the moments of d/dq
-    const float a[9] = { float(-2.0 * (double(M.v[0]) * m[0] + double(M.v[1]) * m[1])), float(-2.0 * (double(M.v[1]) * m[0] + double(M.v[2]) * m[1])),
-        float(m[2]), float(m[3]), float(m[4]), float(m[5]), float(m[6]), float(m[7]), float(m[8]) };
     const float G00 = a[2], G01 = a[3] * 0.5f, G11 = a[4];
     // H = -M G M (2x2 symmetric)
     const float MG00 = M.v[0] * G00 + M.v[1] * G01, MG01 = M.v[0] * G01 + M.v[1] * G11;
