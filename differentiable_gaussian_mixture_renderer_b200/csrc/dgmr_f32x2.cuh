@@ -2,7 +2,8 @@
 // half is the scalar IEEE operation, so the results are the scalar code's bits.
 // A packed operation holds the FP32 pipe for two cycles (measured: 72 TFLOP/s
 // of scalar fma, 74 of packed), so it saves issue slots, not FP32 time: for
-// kernels bound by instruction issue.
+// kernels bound by instruction issue.  The functions below are compared with their
+// scalar forms over every float of their ranges (tests/test_gpu_packed_math.py).
 #pragma once
 
 #include <cstdint>
@@ -48,7 +49,22 @@ __device__ __forceinline__ F2 add2(F2 a, F2 b)
     return r;
 }
 
-// exp_f_nonpos (dgmr_fmath.h) of both halves, for x in [-87, 0]: the 2^n scaling
+// 1 / x of both halves for x in [0.0099, 1]: the approximate reciprocal (within an
+// ulp there) and one Newton step y + y (1 - x y).  The division's result for every
+// float of that range (a test compares all of them).  The division itself carries a
+// slow path for operands that this range never has: the splat backward, with two
+// reciprocals per record and lane, took 324 us instead of 281 with it at 1M, 1080p.
+__device__ __forceinline__ F2 recip2(F2 x)
+{
+    float x0, x1, y0, y1;
+    split2(x, &x0, &x1);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(x0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(x1));
+    const F2 y = f2(y0, y1);
+    return fma2(y, fma2(f2(-x0, -x1), y, f2(1.f)), y);
+}
+
+// exp_f_nonpos (dgmr_fmath.h) of both halves, for x in [-87, 85]: the 2^n scaling
 // as an add to the exponent (the scaled value is normal there, so the product
 // is that bit pattern).
 __device__ __forceinline__ F2 exp2_nonpos(F2 x)

@@ -762,15 +762,8 @@ __device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, f
     al0 = use0 ? al0 : 0.f;
     al1 = use1 ? al1 : 0.f;
     const F2 g = f2(use0 ? e0 : 0.f, use1 ? e1 : 0.f), alpha = f2(al0, al1);
-    // 1 / (1 - alpha), 1 - alpha in [0.01, 1]: the hardware's approximation and
-    // one Newton step y + y (1 - x y), the correctly rounded quotient for every
-    // float in [0.0099, 1] (compared once with the division)
-    const float x0 = 1.f - al0, x1 = 1.f - al1;
-    float y0, y1;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(x0));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(x1));
-    F2 inv = f2(y0, y1);
-    inv = fma2(inv, fma2(f2(-x0, -x1), inv, f2(1.f)), inv);
+    const float x0 = 1.f - al0, x1 = 1.f - al1; // in [0.01, 1]
+    const F2 keep = f2(x0, x1), inv = recip2(keep);
     const F2 Tr = mul2(p.Tr, inv);
     const F2 aT = mul2(alpha, Tr);
     const F2 w0 = mul2(aT, p.g0), w1 = mul2(aT, p.g1), w2 = mul2(aT, p.g2);
@@ -788,7 +781,6 @@ __device__ __forceinline__ bool bwd_record(BwdPixels& p, float4 r0, float4 r1, f
     // d/dcentre = -g_q (2a dx + 2b dy, 2c dy + 2b dx)
     const F2 ux = fma2(f2(-r0.z), f2(dx), mul2(f.x, neg)), uy = fma2(f.y, f2(-2.f), f2(-r1.x * dx));
     const F2 gxx = mul2(gx, f2(dx)), gxy = mul2(mul2(gx, f2(2.f)), dy), gyy = mul2(gy, dy);
-    const F2 keep = f2(x0, x1); // 1 - alpha
     const F2 na0 = add2(mul2_rounded(alpha, f2(c.x)), mul2_rounded(keep, p.a0));
     const F2 na1 = add2(mul2_rounded(alpha, f2(c.y)), mul2_rounded(keep, p.a1));
     const F2 na2 = add2(mul2_rounded(alpha, f2(c.z)), mul2_rounded(keep, p.a2));
