@@ -430,7 +430,8 @@ constexpr int kQuarterWarps = 4;
 // and the ids of the one after are requested before the current batch is
 // worked on.  (Loaded when their batch began, list, record and colour were three
 // latencies in a row, 94 times for the 3000 entries of a slow tile, and the
-// launch waits for its slowest tile.)
+// launch waits for its slowest tile.)  A walk of an empty list requests nothing; in
+// any other, N > 0, and a lane without an entry reads Gaussian 0's record.
 struct ListWalk {
     float4 r0, r1; // of the lane's entry in the next batch
     float c0, c1, c2;
@@ -532,7 +533,8 @@ __global__ void __launch_bounds__(kQuarterWarps * 32, 5) k_splat_blend_quarters(
     Walk next;
     next.id = Walk::entry(list, b + lane, b, e);
     next.later = Walk::entry(list, b + 32 + lane, b, e);
-    next.request(rec, rgb, N);
+    if (b < e)
+        next.request(rec, rgb, N);
     for (int32_t base = b; base < e; base += 32) {
         if (__all_sync(0xffffffffu, p.done0 && p.done1))
             break;
@@ -893,7 +895,8 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 5) k_splat_bwd_pixels(const in
     ListWalk next;
     next.id = ListWalk::entry(list + b, end - 32 + lane, 0, end);
     next.later = ListWalk::entry(list + b, end - 64 + lane, 0, end);
-    next.request(rec, rgb, N);
+    if (end > 0)
+        next.request(rec, rgb, N);
     for (int32_t hi = end; hi > 0; hi -= 32) {
         // the batch's records that can reach a pixel of this quarter (the
         // forward's exact rectangle cull), compacted in list order with their
