@@ -1874,6 +1874,13 @@ extern "C" dgmr_status dgmr_camera_read(const void* view, const void* proj, cons
 {
     if (!view || !proj || !campos || !background || !camera || (dtype != DGMR_F32 && dtype != DGMR_F64))
         return DGMR_ERR_BAD_ARG;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    // refused inside a capture, before anything touches the stream: the wait below would end the capture
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return DGMR_ERR_CUDA;
+    }
     static thread_local CameraStaging staging;
     if (!staging.host
         && cudaHostAlloc(reinterpret_cast<void**>(&staging.host), kCameraValues * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
@@ -1881,7 +1888,6 @@ extern "C" dgmr_status dgmr_camera_read(const void* view, const void* proj, cons
         cudaGetLastError();
         return DGMR_ERR_CUDA;
     }
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (dtype == DGMR_F32)
         k_camera_read<<<1, 64, 0, s>>>(static_cast<const float*>(view), static_cast<const float*>(proj), static_cast<const float*>(campos),
             static_cast<const float*>(background), staging.host);
@@ -1889,8 +1895,10 @@ extern "C" dgmr_status dgmr_camera_read(const void* view, const void* proj, cons
         k_camera_read<<<1, 64, 0, s>>>(static_cast<const double*>(view), static_cast<const double*>(proj), static_cast<const double*>(campos),
             static_cast<const double*>(background), staging.host);
     note_launch();
-    if (launch_status() != DGMR_OK || cudaStreamSynchronize(s) != cudaSuccess)
+    if (launch_status() != DGMR_OK || cudaStreamSynchronize(s) != cudaSuccess) {
+        cudaGetLastError(); // reported here, not by the next call
         return DGMR_ERR_CUDA;
+    }
     std::memcpy(camera->view, staging.host, kCameraValues * sizeof(double));
     return DGMR_OK;
 }

@@ -474,7 +474,8 @@ dgmr_status dgmr_server_destroy(dgmr_server* server);
 /* Reads a camera that lives on the device: view and proj (16 values each),
  * campos and background (3 each), contiguous device arrays of `dtype`
  * (DGMR_F32 / DGMR_F64), into the struct's fields of the same names, and waits for
- * the stream.  One small kernel instead of four copies, each waited for. */
+ * the stream.  One small kernel instead of four copies, each waited for.  Refused
+ * with DGMR_ERR_CUDA on a stream that is being captured, which it leaves as it is. */
 dgmr_status dgmr_camera_read(const void* view, const void* proj, const void* campos, const void* background, int32_t dtype, dgmr_camera* camera,
     dgmr_stream stream);
 
