@@ -1848,13 +1848,30 @@ static_assert(offsetof(dgmr_camera, proj) == offsetof(dgmr_camera, view) + 16 * 
         && offsetof(dgmr_camera, background) == offsetof(dgmr_camera, campos) + 3 * sizeof(double),
     "the four arrays follow one another");
 
+// While it lives, this thread's allocations are no part of a capture that another thread has under way.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // pinned host memory that the kernel writes: one block per thread, kept until the thread ends
 struct CameraStaging {
     double* host = nullptr;
+    cudaError_t allocate(size_t bytes)
+    {
+        const RelaxedCapture relaxed;
+        const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&host), bytes, cudaHostAllocPortable | cudaHostAllocMapped);
+        if (e != cudaSuccess)
+            host = nullptr;
+        return e;
+    }
     ~CameraStaging()
     {
-        if (host)
-            cudaFreeHost(host);
+        if (!host)
+            return;
+        const RelaxedCapture relaxed;
+        cudaFreeHost(host);
     }
 };
 
@@ -1882,9 +1899,7 @@ extern "C" dgmr_status dgmr_camera_read(const void* view, const void* proj, cons
         return DGMR_ERR_CUDA;
     }
     static thread_local CameraStaging staging;
-    if (!staging.host
-        && cudaHostAlloc(reinterpret_cast<void**>(&staging.host), kCameraValues * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-        staging.host = nullptr;
+    if (!staging.host && staging.allocate(kCameraValues * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
         return DGMR_ERR_CUDA;
     }
