@@ -424,7 +424,8 @@ static __global__ void __launch_bounds__(1024) k_chunk_plan(const int32_t* __res
 }
 
 // The same, and the super-tiles' ranges, from the digit totals of a sort whose one
-// pass covered all their bits (digit = super-tile, at most 256): without the
+// pass covered all their bits (digit = super-tile; at most 255, since the sort takes
+// the bits of the count, of which 256 has nine): without the
 // pass over the sorted keys that finds the ranges (k_tile_ranges, 5.7 us for 1.7M
 // entries).  One block of kSortBins threads.
 static __global__ void __launch_bounds__(kSortBins) k_super_plan(const uint32_t* __restrict__ digit_total, uint32_t n_super, int32_t* __restrict__ super_ranges,
