@@ -11,11 +11,14 @@
 //
 // Forward at 10k, 256^2: 0.219 -> 0.173 ms; at 1M, 1080p: 0.577 -> 0.528; forward +
 // backward at 200k, 1024^2: 0.669 -> 0.620 (means of four cameras).  Above
-// kChainMost Gaussian slots the kernels are long enough for the places they hold
-// to cost more than the gaps (12 batched views of 7.4M slots: 5.228 ms plain, 5.241
-// chained), and a blend of more than kChainBlendTiles tiles does not fit the chip
-// at once (chained behind its order kernel: 1M, 1080p 0.540 ms instead of 0.528; at
-// 256 tiles 0.173 instead of 0.180).
+// kChainMost Gaussian slots the kernels over them are long enough for the places
+// they hold to cost more than the gaps (12 batched views of 7.4M slots: 5.228 ms
+// plain, 5.241 chained).  At any size chained (kChainAlways): kernels of one block,
+// which hold one place, and the scan behind a single frame's preprocess (2.5M
+// Gaussians, 1080p: 0.835 ms, plain 0.845; 4M, 1024^2: 0.929, 0.933).  A blend that
+// does not fit the chip at once is launched plainly, and so is its order kernel (1M,
+// 1080p, 8160 tiles: chained 0.540 ms instead of 0.528; at 256 tiles 0.173 instead of
+// 0.180).
 #pragma once
 
 #include <cstdint>
@@ -31,13 +34,13 @@ __device__ __forceinline__ void chain_start()
 }
 
 constexpr uint32_t kChainMost = 2u << 20;
-constexpr uint32_t kChainBlendTiles = 740; // 148 SMs x 5 blocks
+constexpr bool kChainAlways = true;
 
-// A stream, and whether short kernels on it are chained.
+// A stream, and whether a kernel launched on it is chained.
 struct ChainStream {
     cudaStream_t s;
     bool chained;
-    ChainStream(cudaStream_t stream, bool chain = true)
+    ChainStream(cudaStream_t stream, bool chain)
         : s(stream)
         , chained(chain)
     {

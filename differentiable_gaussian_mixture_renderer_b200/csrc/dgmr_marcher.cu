@@ -482,7 +482,7 @@ inline const uint32_t* march_order(const int32_t* ranges, const CameraT<T>& cam,
     if (!workspace || workspace_bytes < off + size_t(n_tiles) * sizeof(uint32_t))
         return nullptr;
     uint32_t* order = reinterpret_cast<uint32_t*>(static_cast<char*>(workspace) + off);
-    launch_chained(k_tile_order, 1, 1024, 0, s, ranges, n_tiles, order);
+    launch_chained(k_tile_order, 1, 1024, 0, ChainStream(s, kChainAlways), ranges, n_tiles, order);
     note_launch();
     return order;
 }
@@ -513,8 +513,8 @@ dgmr_status vm_preprocess(const dgmr_scene* scene, const dgmr_camera* camera, dg
         scene_formulation(scene, Formulation::Opacity) };
     k_vm_preprocess<T><<<(N + 127) / 128, 128, 0, s>>>(p, cam);
     note_launch();
-    inclusive_scan_u32(reinterpret_cast<uint32_t*>(c->tiles_touched), reinterpret_cast<uint32_t*>(c->point_offsets), N, Lw.pre_scan_tmp, s);
-    launch_chained(k_pair_count, 1, 1, 0, s, reinterpret_cast<uint32_t*>(c->point_offsets), N, 0xffffffffu, st_dev, Lw.pre_scan_tmp);
+    inclusive_scan_u32(reinterpret_cast<uint32_t*>(c->tiles_touched), reinterpret_cast<uint32_t*>(c->point_offsets), N, Lw.pre_scan_tmp, ChainStream(s, kChainAlways));
+    launch_chained(k_pair_count, 1, 1, 0, ChainStream(s, kChainAlways), reinterpret_cast<uint32_t*>(c->point_offsets), N, 0xffffffffu, st_dev, Lw.pre_scan_tmp);
     note_launch();
     return launch_status();
 }
@@ -543,7 +543,7 @@ dgmr_status vm_render(const dgmr_scene* scene, const dgmr_camera* camera, dgmr_v
     cudaMemsetAsync(st_dev, 0, 16, s);
     BinningBuffers bin = L.bin;
     if (N > 0)
-        launch_chained(k_depth_keys<T>, (N + 255) / 256, 256, 0, s, static_cast<const T*>(c->depths), N, bin.depth_key, bin.perm);
+        launch_chained(k_depth_keys<T>, (N + 255) / 256, 256, 0, ChainStream(s, N <= kChainMost), static_cast<const T*>(c->depths), N, bin.depth_key, bin.perm);
     if (N > 0)
         note_launch();
     const int par = run_binning<T>(N, cam.gx, cam.gy, reinterpret_cast<uint32_t*>(c->tiles_touched), reinterpret_cast<uint32_t*>(c->point_offsets), c->rects,
@@ -1002,7 +1002,7 @@ dgmr_status dgmr_vm_batch_preprocess(const dgmr_scene* scenes, int32_t n_scenes,
     uint32_t* st_dev = stats ? reinterpret_cast<uint32_t*>(stats) : plan.L.stats;
     vm_batch_preprocess(plan, st_dev, s);
     if (plan.tab.G > 0) {
-        launch_chained(k_pair_count, 1, 1, 0, s, plan.L.point_offsets, plan.tab.G, 0xffffffffu, st_dev, plan.L.bin.n_sort);
+        launch_chained(k_pair_count, 1, 1, 0, ChainStream(s, kChainAlways), plan.L.point_offsets, plan.tab.G, 0xffffffffu, st_dev, plan.L.bin.n_sort);
         note_launch();
     }
     return launch_status();
@@ -1028,7 +1028,7 @@ dgmr_status dgmr_vm_batch_forward(const dgmr_scene* scenes, int32_t n_scenes, co
     vm_batch_preprocess(plan, st_dev, s);
     const int par = run_binning_grids<float>(G, n_tiles, plan.tab.n_stiles, plan.tab, L.tiles_touched, L.point_offsets, L.rects, L.xy, cap, L.bin, L.ranges,
         st_dev, num_sms(), s, true);
-    launch_chained(k_tile_order, 1, 1024, 0, s, L.ranges, n_tiles, L.tile_order);
+    launch_chained(k_tile_order, 1, 1024, 0, ChainStream(s, kChainAlways), L.ranges, n_tiles, L.tile_order);
     const VmMarch<float> a = vm_batch_march(L, L.bin.pair_val[par], st_dev);
     k_vm_march_warp<float, VmBatchFrames><<<n_tiles * (kTilePixels / kRayWarps), kRayWarps * 32, 0, s>>>(a, VmBatchFrames { plan.tab }, L.tile_order);
     note_launch(2);

@@ -225,7 +225,7 @@ void vr_launch_preprocess(const dgmr_scene* scene, const CameraT<float>& cam, co
         ((kVrFilterSD * cam.tan_fovx) * 2.f) / float(cam.W), scene_formulation(scene, Formulation::Ots) };
     k_vr_preprocess<<<(N + 127) / 128, 128, 0, s>>>(p, cam);
     note_launch();
-    inclusive_scan_u32(L.tiles_touched, L.point_offsets, N, L.bin.scan_tmp, s);
+    inclusive_scan_u32(L.tiles_touched, L.point_offsets, N, L.bin.scan_tmp, ChainStream(s, kChainAlways));
 }
 
 } // namespace
@@ -259,7 +259,7 @@ dgmr_status dgmr_vr_preprocess(const dgmr_scene* scene, const dgmr_camera* camer
     uint32_t* st_dev = stats ? reinterpret_cast<uint32_t*>(stats) : L.stats;
     vr_launch_preprocess(scene, cam, L, st_dev, s);
     if (scene->n_gaussians > 0) {
-        launch_chained(k_pair_count, 1, 1, 0, s, L.point_offsets, uint32_t(scene->n_gaussians), 0xffffffffu, st_dev, L.bin.n_sort);
+        launch_chained(k_pair_count, 1, 1, 0, ChainStream(s, kChainAlways), L.point_offsets, uint32_t(scene->n_gaussians), 0xffffffffu, st_dev, L.bin.n_sort);
         note_launch();
     }
     return launch_status();

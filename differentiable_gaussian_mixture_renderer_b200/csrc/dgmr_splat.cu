@@ -282,13 +282,17 @@ struct SingleFrame {
     __device__ __forceinline__ FrameRef frame(uint32_t tile) const { return FrameRef { W, H, gx, tile, bg0, bg1, bg2, fb, final_T, n_contrib, grad_fb }; }
 };
 
+// Blocks of either blend kernel on an SM; a block is a tile.
+constexpr int kBlendBlocks = 5;
+inline bool blend_fits_chip(uint32_t n_tiles) { return n_tiles <= uint32_t(num_sms()) * kBlendBlocks; }
+
 // The blend with a 16x16 tile per block of 256 threads, a pixel each (batches may
 // choose it, dgmr_batch_view.blend_block; the same bits as the quarters below).
 // __launch_bounds__ keeps it at 48 registers, five blocks per SM instead of four at
 // the 52 the compiler picks unbounded: 3 % shorter launches over 8 cameras at
 // 1080p/1M.
 template <class Frames>
-__global__ void __launch_bounds__(kTilePixels, 5) k_splat_blend_tiles(const int32_t* __restrict__ ranges, const uint32_t* __restrict__ list,
+__global__ void __launch_bounds__(kTilePixels, kBlendBlocks) k_splat_blend_tiles(const int32_t* __restrict__ ranges, const uint32_t* __restrict__ list,
     const float4* __restrict__ rec, const float* __restrict__ rgb, uint32_t N, uint32_t cap, uint32_t* __restrict__ stats,
     const uint32_t* __restrict__ tile_order, const __grid_constant__ Frames frames)
 {
@@ -504,7 +508,7 @@ __device__ __forceinline__ void blend_record2(QuarterPixels& p, F2 q, F2 ex, boo
 }
 
 template <class Frames>
-__global__ void __launch_bounds__(kQuarterWarps * 32, 5) k_splat_blend_quarters(const int32_t* __restrict__ ranges, const uint32_t* __restrict__ list,
+__global__ void __launch_bounds__(kQuarterWarps * 32, kBlendBlocks) k_splat_blend_quarters(const int32_t* __restrict__ ranges, const uint32_t* __restrict__ list,
     const float4* __restrict__ rec, const float* __restrict__ rgb, uint32_t N, uint32_t cap, uint32_t* __restrict__ stats,
     const uint32_t* __restrict__ tile_order, const __grid_constant__ Frames frames)
 {
@@ -648,9 +652,9 @@ void launch_blend(int side, uint32_t n_tiles, const int32_t* ranges, const uint3
     if (n_tiles == 0)
         return;
     if (side == 8)
-        launch_chained(k_splat_blend_quarters<Frames>, n_tiles, kQuarterWarps * 32, 0, ChainStream(s, n_tiles <= kChainBlendTiles), ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
+        launch_chained(k_splat_blend_quarters<Frames>, n_tiles, kQuarterWarps * 32, 0, ChainStream(s, blend_fits_chip(n_tiles)), ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
     else
-        launch_chained(k_splat_blend_tiles<Frames>, n_tiles, kTilePixels, 0, ChainStream(s, n_tiles <= kChainBlendTiles), ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
+        launch_chained(k_splat_blend_tiles<Frames>, n_tiles, kTilePixels, 0, ChainStream(s, blend_fits_chip(n_tiles)), ranges, list, rec, rgb, N, cap, stats, tile_order, frames);
     note_launch();
 }
 
@@ -1156,7 +1160,7 @@ void launch_preprocess(const dgmr_scene* scene, const CameraT<float>& cam, const
         return;
     k_splat_preprocess<<<(N + 255) / 256, 256, 0, s>>>(make_pre(scene, L), cam);
     note_launch();
-    inclusive_scan_u32(L.tiles_touched, L.point_offsets, N, L.bin.scan_tmp, s);
+    inclusive_scan_u32(L.tiles_touched, L.point_offsets, N, L.bin.scan_tmp, ChainStream(s, kChainAlways));
 }
 
 // Launch order of the blend's tiles, heaviest first, from a predicted cost
@@ -1328,7 +1332,7 @@ void launch_tile_order(const SplatLayout& L, int par, uint32_t N, uint32_t cap, 
     if (n_tiles == 0)
         return;
     launch_chained(k_blend_tile_order<Frames>, (n_tiles + kOrderWarps - 1) / kOrderWarps, kOrderWarps * 32, 0,
-        ChainStream(s, n_tiles <= kChainBlendTiles), L.ranges, L.bin.pair_val[par], L.blend_rec, N, cap,
+        ChainStream(s, blend_fits_chip(n_tiles)), L.ranges, L.bin.pair_val[par], L.blend_rec, N, cap,
         n_tiles, L.tile_cost, L.bin.n_sort + 6, L.tile_order, frames);
     note_launch();
 }
@@ -1404,7 +1408,7 @@ dgmr_status dgmr_splat_preprocess(const dgmr_scene* scene, const dgmr_camera* ca
     uint32_t* st_dev = stats ? reinterpret_cast<uint32_t*>(stats) : L.stats;
     launch_preprocess(scene, cam, L, st_dev, s);
     if (scene->n_gaussians > 0) {
-        launch_chained(k_pair_count, 1, 1, 0, s, L.point_offsets, uint32_t(scene->n_gaussians), 0xffffffffu, st_dev, L.bin.n_sort);
+        launch_chained(k_pair_count, 1, 1, 0, ChainStream(s, kChainAlways), L.point_offsets, uint32_t(scene->n_gaussians), 0xffffffffu, st_dev, L.bin.n_sort);
         note_launch();
     }
     return launch_status();
@@ -1682,7 +1686,7 @@ dgmr_status dgmr_splat_batch_preprocess(const dgmr_scene* scenes, int32_t n_scen
     uint32_t* st_dev = stats ? reinterpret_cast<uint32_t*>(stats) : plan.L.stats;
     batch_preprocess(plan, st_dev, s);
     if (plan.tab.G > 0) {
-        launch_chained(k_pair_count, 1, 1, 0, s, plan.L.point_offsets, plan.tab.G, 0xffffffffu, st_dev, plan.L.bin.n_sort);
+        launch_chained(k_pair_count, 1, 1, 0, ChainStream(s, kChainAlways), plan.L.point_offsets, plan.tab.G, 0xffffffffu, st_dev, plan.L.bin.n_sort);
         note_launch();
     }
     return launch_status();
