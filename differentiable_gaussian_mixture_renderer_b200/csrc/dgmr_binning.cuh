@@ -787,7 +787,8 @@ static __global__ void __launch_bounds__(kChunkThreads) k_chunk_emit(const uint3
     }
 }
 
-inline size_t chunk_emit_smem() { return size_t(kEmitStage) * (sizeof(uint32_t) + sizeof(uint8_t)); }
+constexpr size_t chunk_emit_smem() { return size_t(kEmitStage) * (sizeof(uint32_t) + sizeof(uint8_t)); }
+static_assert(chunk_emit_smem() <= 40 * 1024, "with the kernel's 6 KB of static arrays within the 48 KB that need no opt-in");
 
 // [start, end) of every run of equal keys in a sorted key list (the tile
 // ranges of splat_forward.cu:218-239; here applied to the sorted super-tile
@@ -933,11 +934,6 @@ inline int run_binning_grids(uint32_t N, uint32_t n_tiles, uint32_t n_super, con
             inclusive_scan_u32(b.tile_total, b.tile_incl, n_tiles, b.scan_tmp, s);
             launch_chained(k_tile_ranges_from_counts, (n_tiles + 255) / 256, 256, 0, s, b.tile_total, b.tile_incl, n_tiles, cap, ranges);
             note_launch();
-        }
-        static bool smem_set = false; // one opt-in per instantiation, above the 48 KB default
-        if (!smem_set) {
-            cudaFuncSetAttribute(k_chunk_emit<Grids>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(chunk_emit_smem()));
-            smem_set = true;
         }
         launch_chained(k_chunk_emit<Grids>, cgrid, kChunkThreads, chunk_emit_smem(), s, b.pair_tile[spar], b.pair_val[spar], N, b.super_ranges, b.chunk_base, n_super,
             b.n_sort, rows, b.tile_total, b.tile_incl, cap, keep_tiles ? b.pair_tile[1 - spar] : nullptr, b.pair_val[1 - spar], stats, grids);
