@@ -692,10 +692,12 @@ __device__ __forceinline__ float warp_reduce_scatter12(const float (&v)[12], int
 // by one warp reduction.  Each pixel walks its contributors back to front,
 // recovering T_i = T_{i+1} / (1 - alpha_i).  Per record the warp sums the
 // gradients of the centre, the conic, the opacity and the colour over its pixels,
-// and twelve lanes add one value each.  A float sum covers 32 pixels, the even or
-// the odd columns of the quarter, which meet in double; the conic's three cover
-// 16, upper and lower half apart: the chain to a long thin splat's scales cancels
-// by 10^5, and with float sums over 64 pixels single elements moved by 1e-3.  The
+// and eighteen lanes add one value each.  A float sum covers 32 pixels, which meet in
+// double: for the conic the upper or the lower half of the quarter, for the others
+// its even or its odd columns.  The chain from the conic to a long thin splat's
+// scales cancels by 10^5; with float sums over 64 pixels single elements moved by
+// 1e-3, and grouped as the others (16 pixels at a time then) they are closer to the
+// exact sums but move by up to 2e-2 on splats 30 to 1000 times as long as wide.  The
 // totals over warps are double too: in float, the order in which the atomics of
 // many cancelling terms land moved single elements by ~1e-3 relative from run to
 // run at 200k Gaussians, 1024^2.
@@ -713,7 +715,7 @@ __device__ __forceinline__ float warp_reduce_scatter12(const float (&v)[12], int
 // 80 registers without spills beat 64 with them, and the next batch is requested
 // ahead (ListWalk: 299 -> 273 us at 1M, 1080p, 284 -> 288 at 200k, 1024^2).  Against a
 // pixel per lane, a reduction per 32 pixels of all nine values and 48 registers:
-// 401 -> 281 us at 1M, 1080p; 430 -> 299 us at 200k, 1024^2.
+// 401 -> 282 us at 1M, 1080p; 430 -> 304 us at 200k, 1024^2.
 constexpr int kBwdWarps = 4; // the quarters of a tile
 static_assert(kTile == 16, "four 8x8 quarters per tile");
 
@@ -890,11 +892,13 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 5) k_splat_bwd_pixels(const in
     // the accumulator of each reduced slot: 0, 1, then the conic's three from both halves, then opacity and colour
     const int slot = reduce_slot(lane);
     const int my_slot = slot < 2 ? slot : slot < 8 ? 1 + slot / 2 : slot - 3;
-    const bool adds = (lane & 1) == 0 && ((lane & 2) == 0 || (lane & 4) == 0); // slot 2 of three is on both lanes of bit 2
+    const bool conic = slot >= 2 && slot < 8; // its lanes of both parities add up in float, and the even one adds the sum
+    const bool adds = ((lane & 1) == 0 || !conic) && ((lane & 2) == 0 || (lane & 4) == 0); // slot 2 of three is on both lanes of bit 2
     const auto add = [&](float part) {
-        const double total = double(part) + double(__shfl_xor_sync(0xffffffffu, part, 1));
-        if (adds && held_id != 0xffffffffu && total != 0.0)
-            atomicAdd(acc + size_t(held_id) * 9 + my_slot, total);
+        const float other = __shfl_xor_sync(0xffffffffu, part, 1);
+        const float sum = conic ? part + other : part;
+        if (adds && held_id != 0xffffffffu && sum != 0.f)
+            atomicAdd(acc + size_t(held_id) * 9 + my_slot, double(sum));
     };
     ListWalk next;
     next.id = ListWalk::entry(list + b, end - 32 + lane, 0, end);
