@@ -269,7 +269,8 @@ __device__ __forceinline__ bool plain_record(float4 r0, float4 r1, float4 rgb, f
 // The kernel's duration is set by its slowest tile (a few tiles with ~2-3k
 // unsaturated entries run from the first wave to the end), so a tile's
 // pixels are spread over as many threads as it has pixels: two pixels per
-// thread made that critical path, and the launch, 12 % longer.
+// thread, evaluated one after the other, made that critical path, and the launch,
+// 12 % longer.  (The quarters below take two per thread in packed instructions.)
 
 // A single frame: every tile is one of its tiles.
 struct SingleFrame {
@@ -712,7 +713,7 @@ __device__ __forceinline__ float warp_reduce_scatter12(const float (&v)[12], int
 //
 // Bound by instruction issue, and at the end of a launch by the longest warp's
 // serial walk: so a record's reduction is issued with the next record's body, and
-// 80 registers without spills beat 64 with them, and the next batch is requested
+// 89 registers without spills beat 64 with them, and the next batch is requested
 // ahead (ListWalk: 299 -> 273 us at 1M, 1080p, 284 -> 288 at 200k, 1024^2).  Against a
 // pixel per lane, a reduction per 32 pixels of all nine values and 48 registers:
 // 401 -> 282 us at 1M, 1080p; 430 -> 304 us at 200k, 1024^2.
